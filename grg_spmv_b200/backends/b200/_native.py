@@ -15,14 +15,15 @@ import threading
 PACKAGE_DIR = Path(__file__).resolve().parents[2]
 REPO_DIR = PACKAGE_DIR.parent
 LIB_PATH = PACKAGE_DIR / "libgrg_b200.so"
-SOURCES = (PACKAGE_DIR / "csrc" / "grg_b200.cu",)
+SOURCES = (PACKAGE_DIR / "csrc" / "grg_b200.cu", PACKAGE_DIR / "csrc" / "level_walk.cu")
+OBJECT_DIR = PACKAGE_DIR / "_build"
 HEADER_DIR = REPO_DIR / "include"
-ABI_VERSION = 14
+ABI_VERSION = 15
 
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
 )
 
 # Status codes, enums and entry coding (grg_b200.h).
@@ -30,6 +31,9 @@ OK, ERR_INVALID, ERR_CUDA, ERR_UNSUPPORTED = 0, 1, 2, 3
 F64, F32, MIXED = 0, 1, 2
 MAX_SLOT_BUCKETS = 8
 LAUNCH_PDL = 1
+LAUNCH_WALK = 2
+LONG_ROW = 512
+LONG_CLASSES = 8
 SCHEDULE_LEVELS, SCHEDULE_DATAFLOW = 0, 1
 DEVICE_WAIT_TIMEOUT = 6
 UP, DOWN = 0, 1
@@ -80,6 +84,7 @@ class Level(ctypes.Structure):
         ("slot_entry", ctypes.c_int64 * 8),
         ("slot_width", ctypes.c_int32 * 8),
         ("short_rows", ctypes.c_int64),
+        ("long_rows", ctypes.c_int64 * LONG_CLASSES),
     ]
 
 
@@ -191,16 +196,34 @@ _lib = None
 
 
 def build_library(*, force: bool = False, verbose: bool = False) -> Path:
-    """Compile ``libgrg_b200.so`` for sm_100a with nvcc (cross-compiles without a GPU)."""
-    newest = max(p.stat().st_mtime for p in (*SOURCES, HEADER_DIR / "grg_b200.h"))
+    """Compile ``libgrg_b200.so`` for sm_100a with nvcc (cross-compiles without a GPU): one
+    object per source, side by side, then the link."""
+    headers = max(p.stat().st_mtime for p in (*SOURCES[0].parent.glob("*.h"), *SOURCES[0].parent.glob("*.cuh"), HEADER_DIR / "grg_b200.h"))
+    newest = max(headers, *(p.stat().st_mtime for p in SOURCES))
     if not force and LIB_PATH.exists() and LIB_PATH.stat().st_mtime >= newest:
         return LIB_PATH
     nvcc = os.environ.get("NVCC", "nvcc")
+    OBJECT_DIR.mkdir(exist_ok=True)
+    running, objects = [], []
+    for source in SOURCES:
+        obj = OBJECT_DIR / f"{source.stem}.o"
+        objects.append(obj)
+        if not force and obj.exists() and obj.stat().st_mtime >= max(headers, source.stat().st_mtime):
+            continue
+        cmd = [nvcc, *NVCC_FLAGS, f"-I{HEADER_DIR}", "-c", "-o", str(obj) + ".tmp", str(source)]
+        if verbose:
+            cmd.insert(1, "-Xptxas=-v")
+        running.append((obj, cmd, subprocess.Popen(cmd)))
+    failed = None
+    for obj, cmd, process in running:
+        if process.wait() != 0:
+            failed = subprocess.CalledProcessError(process.returncode, cmd)
+        else:
+            Path(str(obj) + ".tmp").replace(obj)
+    if failed is not None:
+        raise failed
     tmp = LIB_PATH.with_suffix(".so.tmp")
-    cmd = [nvcc, *NVCC_FLAGS, f"-I{HEADER_DIR}", "-o", str(tmp), *map(str, SOURCES)]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    subprocess.run(cmd, check=True)
+    subprocess.run([nvcc, *NVCC_FLAGS, "-shared", "-o", str(tmp), *map(str, objects)], check=True)
     tmp.replace(LIB_PATH)
     return LIB_PATH
 

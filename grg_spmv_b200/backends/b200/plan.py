@@ -62,8 +62,10 @@ class B200Plan:
     ``row_order``: "natural" (node order) or "locality" (rows that share source rows are
     processed together); None picks the direction's default (up natural, down locality).
     ``narrow_variant``: shape of the narrow-row kernel (``GRG_B200_NARROW_VARIANTS``); None
-    picks per call, as measured on B200: in the default mode the lean entry-parallel walk in
-    4-warp CTAs, 15 (run as 12 where its shape does not apply: k not a power of two, or above 64 in FP64 and
+    picks per call, as measured on B200: in the default mode the walk that the library chooses
+    per level (``GRG_B200_LAUNCH_WALK``; not with a ``heavy_variant`` or ``narrow_split`` of one's
+    own), and for launches it does not serve (an init inside the traversal, bounds checks) the
+    lean entry-parallel walk in 4-warp CTAs, 15 (run as 12 where its shape does not apply: k not a power of two, or above 64 in FP64 and
     128 in FP32); in exact
     order 7 for k <= 16 and 6 above; with ``pad_lists=False``, 5.  Runtimes with bounds
     checking run 7 in place of 11-14.
@@ -79,7 +81,8 @@ class B200Plan:
     ``long_first``: with ``balance``, the longest length bucket is processed first.
     ``pdl``: launch the level, seed and output kernels with programmatic dependent launch
     (each overlaps the end of the previous one; ignored when levels are streamed).  None turns
-    it on for k >= 8: measured on B200, +3% to +4.5% at k = 8, +1% at k = 32, -15% at k = 1.
+    it on for k >= 8, and for every k where the library chooses the row walk (measured on B200,
+    1.5M nodes, k = 1: up 178 -> 160 us, down 197 -> 153 us).
     ``slots``: with ``balance`` and ``pad_lists``, pad each narrow row to its bucket's width
     (1, 2, 4, 8 quads of 4 entries) so kernels locate its list from its position instead of
     loading ``row_ptr`` (one dependent load fewer per row, up to twice the list bytes).
@@ -159,6 +162,12 @@ class B200Plan:
         # one vector per lane, +9.5% over 7 at k = 1 and +8.4% over 12 at k = 2; the same walk
         # in 4-warp CTAs (15) a further +1.9% at k = 8, +2.7% at k = 32, +0.9% at k = 1
         return 15
+
+    def library_walk(self) -> bool:
+        """Whether the library chooses the row walk of each level (``GRG_B200_LAUNCH_WALK``): when
+        nothing in the plan asks for a kernel shape of its own."""
+        return (self.narrow_variant is None and self.heavy_variant is None and int(self.narrow_split) == -1 and self.pad_lists
+                and not self.exact_order)
 
     def resolve_pdl(self, k: int) -> bool:
         """Whether calls with ``k`` right-hand sides use programmatic dependent launch."""

@@ -350,7 +350,8 @@ class B200Runtime:
                                num_heavy=int(lv.heavy_rows.size), heavy_threshold=lv.heavy_threshold, ring_slot=slot,
                                blob=blob.data_ptr(), blob_bytes=nbytes, off_row_ptr=off_ptr, off_heavy=off_heavy,
                                off_row_ids=off_ids, off_entries=off_entries, list_align=lv.list_align,
-                               short_rows=lv.short_rows() if short_rows else 0)
+                               short_rows=lv.short_rows() if short_rows else 0,
+                               long_rows=(ctypes.c_int64 * nat.LONG_CLASSES)(*lv.long_rows()))
             if lv.slots is not None:
                 arr[i].num_slot_buckets = int(lv.slots.shape[0])
                 for b, (pos, entry, width) in enumerate(lv.slots):
@@ -510,6 +511,8 @@ class B200Runtime:
         a.persist_ctas = int(plan.persist_ctas)
         a.fuse_entries = int(plan.fuse_entries)
         a.launch_flags = nat.LAUNCH_PDL if plan.resolve_pdl(k) else 0
+        if plan.library_walk() and direction not in self._variant:
+            a.launch_flags |= nat.LAUNCH_WALK | (nat.LAUNCH_PDL if plan.pdl is None else 0)
         a.schedule = nat.SCHEDULE_DATAFLOW if plan.schedule == "dataflow" else nat.SCHEDULE_LEVELS
         a.dataflow_sync = _ptr(self._df_sync if df_sync is None else df_sync)
         return a

@@ -69,7 +69,7 @@ class LevelGather:
     num_rows: int
     row_ptr: np.ndarray  # int32 [num_rows + 1], by processing position
     entries: np.ndarray  # uint32
-    heavy_rows: np.ndarray  # int32 processing positions
+    heavy_rows: np.ndarray  # int32 processing positions, the longest classes (long_rows) first
     heavy_threshold: int
     row_ids: np.ndarray | None = None  # int32 level-local row of each position (None: identity)
     list_align: int = 1  # 4: lists padded to multiples of 4 entries with null codes
@@ -92,6 +92,12 @@ class LevelGather:
             return 0
         longer = np.flatnonzero(np.diff(self.row_ptr[:narrow + 1].astype(np.int64)) > 4)
         return narrow - (int(longer[-1]) + 1 if longer.size else 0)
+
+    def long_rows(self) -> list[int]:
+        """How many heavy rows hold more than ``LONG_ROW << i`` entries: the first so many of
+        ``heavy_rows``, which kernels may split further than the others."""
+        lengths = self.row_ptr[self.heavy_rows + 1].astype(np.int64) - self.row_ptr[self.heavy_rows]
+        return [int((lengths > (nat.LONG_ROW << i)).sum()) for i in range(nat.LONG_CLASSES)]
 
     def layout(self) -> tuple[int, int, int, int, int]:
         return blob_layout(self.num_rows, self.heavy_rows.size, self.entries.size, self.row_ids is not None)
@@ -141,6 +147,18 @@ def _quad_class(counts: np.ndarray) -> np.ndarray:
     while np.any(width < quads):
         width = np.where(width < quads, width * 2, width)
     return np.where(quads == 0, 0, width)
+
+
+def _heavy_rows(row_ptr: np.ndarray, num_rows: int, num_heavy: int) -> np.ndarray:
+    """The heavy positions (the suffix), those in the longest classes of ``long_rows`` first and
+    in processing order inside a class."""
+    first = num_rows - num_heavy
+    lengths = np.diff(row_ptr[first:].astype(np.int64))
+    long_class = np.searchsorted(_LONG, lengths, side="left")  # lengths above LONG_ROW << i, counted over i
+    return (first + np.argsort(-long_class, kind="stable")).astype(np.int32)
+
+
+_LONG = np.asarray([nat.LONG_ROW << i for i in range(nat.LONG_CLASSES)], dtype=np.int64)
 
 
 def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np.ndarray, src: np.ndarray,
@@ -225,7 +243,7 @@ def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np
         entries, row_ptr = out, new_ptr
         if row_ptr[-1] > np.iinfo(np.int32).max:
             raise ValueError(f"level {level} has {int(row_ptr[-1])} padded entries, above the 2^31-1 per-level limit")
-    heavy = np.arange(num_rows - num_heavy, num_rows, dtype=np.int32)
+    heavy = _heavy_rows(row_ptr, num_rows, num_heavy)
     if slot_table is not None and slot_table.shape[0] > nat.MAX_SLOT_BUCKETS:
         slot_table = None  # more width classes than the kernels take: row_ptr is still exact
     return LevelGather(level, int(row_begin), int(num_rows), row_ptr.astype(np.int32), entries, heavy,
@@ -332,8 +350,9 @@ def _finish_torch(level: int, row_begin: int, num_rows: int, rows: np.ndarray, i
             raise ValueError(f"level {level} has {int(row_ptr[-1])} padded entries, above the 2^31-1 per-level limit")
     if slot_table is not None and slot_table.shape[0] > nat.MAX_SLOT_BUCKETS:
         slot_table = None
-    heavy = np.arange(n - num_heavy, n, dtype=np.int32)
-    return LevelGather(level, int(row_begin), n, row_ptr.to(torch.int32).cpu().numpy(),
+    row_ptr = row_ptr.to(torch.int32).cpu().numpy()
+    heavy = _heavy_rows(row_ptr, n, num_heavy)
+    return LevelGather(level, int(row_begin), n, row_ptr,
                        entries.cpu().numpy().astype(np.uint32), heavy, int(heavy_threshold),
                        None if row_ids is None else row_ids.to(torch.int32).cpu().numpy(), 4 if pad else 1, slot_table)
 

@@ -33,13 +33,16 @@
 #include <mutex>
 #include <type_traits>
 
-#include "grg_b200.h"
+#include "level_common.cuh"
+#include "level_walk.h"
 
 namespace {
 
 thread_local char g_last_error[1024] = "";
 
-int fail(int code, const char* fmt, ...) {
+}  // namespace
+
+int grg_fail(int code, const char* fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_last_error, sizeof(g_last_error), fmt, ap);
@@ -47,243 +50,7 @@ int fail(int code, const char* fmt, ...) {
     return code;
 }
 
-#define GRG_CUDA_TRY(expr)                                                                  \
-    do {                                                                                    \
-        cudaError_t err__ = (expr);                                                         \
-        if (err__ != cudaSuccess)                                                           \
-            return fail(GRG_B200_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(err__)); \
-    } while (0)
-
-#define GRG_LAUNCH_CHECK(name)                                                              \
-    do {                                                                                    \
-        cudaError_t err__ = cudaGetLastError();                                             \
-        if (err__ != cudaSuccess)                                                           \
-            return fail(GRG_B200_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(err__)); \
-    } while (0)
-
-// Launch with programmatic dependent launch when `pdl` (the kernel must call pdl_wait()
-// before touching data that earlier kernels of the stream produce).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_k(bool pdl, cudaStream_t s, dim3 grid, int block, void (*kernel)(KArgs...), Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(static_cast<unsigned>(block));
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-// ---------------------------------------------------------------------------------------
-// Vector packs
-// ---------------------------------------------------------------------------------------
-template <typename T, int V>
-struct alignas(sizeof(T) * V) Pack {
-    T v[V];
-};
-
-template <typename T, int V>
-__device__ __forceinline__ Pack<T, V> zero_pack() {
-    Pack<T, V> r;
-#pragma unroll
-    for (int i = 0; i < V; ++i) r.v[i] = T(0);
-    return r;
-}
-
-template <typename T, int V>
-__device__ __forceinline__ Pack<T, V> splat(T x) {
-    Pack<T, V> r;
-#pragma unroll
-    for (int i = 0; i < V; ++i) r.v[i] = x;
-    return r;
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void add_into(Pack<T, V>& a, const Pack<T, V>& b) {
-#pragma unroll
-    for (int i = 0; i < V; ++i) a.v[i] = a.v[i] + b.v[i];
-}
-
-// Read-only (non-coherent) load: every row read by a kernel was written by an earlier launch.
-template <typename T, int V>
-__device__ __forceinline__ Pack<T, V> ld_ro(const T* p) {
-    Pack<T, V> r;
-    if constexpr (V == 1) {
-        r.v[0] = __ldg(p);
-    } else if constexpr (std::is_same<T, double>::value && V == 2) {
-        const double2 d = __ldg(reinterpret_cast<const double2*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-    } else if constexpr (std::is_same<T, float>::value && V == 2) {
-        const float2 d = __ldg(reinterpret_cast<const float2*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-    } else {
-        static_assert(std::is_same<T, float>::value && V == 4, "unsupported pack");
-        const float4 d = __ldg(reinterpret_cast<const float4*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-        r.v[2] = d.z;
-        r.v[3] = d.w;
-    }
-    return r;
-}
-
-// L2 load (rows written by other SMs during this launch must not come from a stale L1 line).
-template <typename T, int V>
-__device__ __forceinline__ Pack<T, V> ld_l2(const T* p) {
-    Pack<T, V> r;
-    if constexpr (V == 1) {
-        r.v[0] = __ldcg(p);
-    } else if constexpr (std::is_same<T, double>::value && V == 2) {
-        const double2 d = __ldcg(reinterpret_cast<const double2*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-    } else if constexpr (std::is_same<T, float>::value && V == 2) {
-        const float2 d = __ldcg(reinterpret_cast<const float2*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-    } else {
-        const float4 d = __ldcg(reinterpret_cast<const float4*>(p));
-        r.v[0] = d.x;
-        r.v[1] = d.y;
-        r.v[2] = d.z;
-        r.v[3] = d.w;
-    }
-    return r;
-}
-
-// Source-row load of the level walkers: the read-only path, or L2 only (CG) where rows read
-// here may have been written by other SMs earlier in the same launch.
-template <typename T, int V, bool CG>
-__device__ __forceinline__ Pack<T, V> ld_src(const T* p) {
-    if constexpr (CG) return ld_l2<T, V>(p);
-    else return ld_ro<T, V>(p);
-}
-
-template <typename T, int V>
-__device__ __forceinline__ void st_pack(T* p, const Pack<T, V>& x) {
-    *reinterpret_cast<Pack<T, V>*>(p) = x;
-}
-
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-
-// ---------------------------------------------------------------------------------------
-// Kernel parameters
-// ---------------------------------------------------------------------------------------
-struct LevelArgs {
-    int64_t row_begin;
-    int64_t num_rows;
-    const int32_t* row_ptr;
-    const uint32_t* entries;
-    const int32_t* heavy_rows;
-    const int32_t* row_ids;
-    int64_t num_heavy;
-    int32_t heavy_threshold;
-    int32_t list_align;
-    int32_t use_miss;
-    void* state;
-    int64_t ld_state;
-    const void* x;
-    int64_t ld_x;
-    const void* miss;
-    int64_t ld_miss;
-    const void* init_vector;
-    const void* init_matrix;
-    int64_t ld_init;
-    const int32_t* node_perm;
-    const void* xtx_node;
-    int64_t k;
-    int32_t log2g;
-    int32_t* err;
-    int64_t lim_state;
-    int64_t lim_x;
-    int64_t lim_miss;
-    int32_t log2s;  // narrow rows split over 2^log2s lane groups (default mode, variant 6)
-    int32_t num_slot_buckets;  // > 0: narrow lists located from the slot table, not row_ptr
-    int32_t slot_width[GRG_B200_MAX_SLOT_BUCKETS];
-    int64_t slot_pos[GRG_B200_MAX_SLOT_BUCKETS];
-    int64_t slot_entry[GRG_B200_MAX_SLOT_BUCKETS];
-    // mixed storage only: the 16-bit planes of state, x and miss (x/miss hold encoded copies)
-    void* state_lo;
-    const void* x_lo;
-    const void* miss_lo;
-    int32_t up;  // an up level: its lists name state rows (and null padding) only
-    int64_t short_rows;  // entry kernels: the last short_rows narrow positions take one entry slot
-};
-
-enum DeviceError : int32_t {
-    kErrStateId = 1,
-    kErrInputId = 2,
-    kErrMissId = 3,
-    kErrPerm = 4,
-    kErrSelector = 5,
-    kErrWaitTimeout = 6,  // dataflow: a source row never became ready within the spin limit
-};
-
-__device__ __forceinline__ void report(int32_t* err, int32_t code) {
-    if (err) atomicCAS(err, 0, code);
-}
-
-// Programmatic dependent launch: a kernel launched with it may start while the previous
-// kernel of the stream is finishing; it reads only static data (level lists) until
-// pdl_wait(), which returns once the previous grid has completed and its writes are visible
-// (immediately when the launch did not use the attribute).  pdl_trigger() lets the next
-// kernel launch once every CTA of this grid has started.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
-
-template <typename T, int V, int INIT>
-__device__ __forceinline__ Pack<T, V> init_value(const LevelArgs& a, int64_t row, int64_t c) {
-    if constexpr (INIT == GRG_B200_INIT_VECTOR) {
-        return ld_ro<T, V>(static_cast<const T*>(a.init_vector) + c);
-    } else if constexpr (INIT == GRG_B200_INIT_XTX) {
-        return splat<T, V>(__ldg(static_cast<const T*>(a.xtx_node) + row));
-    } else if constexpr (INIT == GRG_B200_INIT_MATRIX) {
-        const int64_t orig = __ldg(a.node_perm + row);
-        if (a.err && (orig < 0 || orig >= a.lim_state)) {
-            report(a.err, kErrPerm);
-            return zero_pack<T, V>();
-        }
-        return ld_ro<T, V>(static_cast<const T*>(a.init_matrix) + orig * a.ld_init + c);
-    } else {
-        return zero_pack<T, V>();
-    }
-}
-
-// Address of the row named by a coded entry; nullptr when the entry is skipped.
-template <typename T>
-__device__ __forceinline__ const T* entry_row(const LevelArgs& a, uint32_t code) {
-    const uint32_t src = (code >> GRG_B200_SRC_SHIFT) & GRG_B200_SRC_MASK;
-    const int64_t id = code & GRG_B200_ID_MASK;
-    if (src == GRG_B200_SRC_STATE) {
-        if (a.err && id >= a.lim_state) {
-            report(a.err, kErrStateId);
-            return nullptr;
-        }
-        return static_cast<const T*>(a.state) + id * a.ld_state;
-    }
-    if (src == GRG_B200_SRC_INPUT) {
-        if (a.err && id >= a.lim_x) {
-            report(a.err, kErrInputId);
-            return nullptr;
-        }
-        return static_cast<const T*>(a.x) + id * a.ld_x;
-    }
-    if (src != GRG_B200_SRC_MISS || !a.use_miss) return nullptr;  // null padding, or miss rows off
-    if (a.err && id >= a.lim_miss) {
-        report(a.err, kErrMissId);
-        return nullptr;
-    }
-    return static_cast<const T*>(a.miss) + id * a.ld_miss;
-}
+namespace {
 
 // ---------------------------------------------------------------------------------------
 // Level kernels
@@ -291,11 +58,6 @@ __device__ __forceinline__ const T* entry_row(const LevelArgs& a, uint32_t code)
 constexpr int kNarrowThreads = 256;
 constexpr int kNarrowWarps = kNarrowThreads / 32;
 constexpr int kStageCap = 1024;  // gather-list entries staged in shared memory per warp
-constexpr unsigned kFullMask = 0xffffffffu;
-
-__device__ __forceinline__ int64_t level_row(const LevelArgs& a, int64_t pos) {
-    return a.row_begin + (a.row_ids ? static_cast<int64_t>(__ldg(a.row_ids + pos)) : pos);
-}
 
 // Narrow rows.  A warp owns 32/G consecutive processing positions; lane group g (G lanes)
 // owns position g and columns [lane*V, lane*V + V) (+ multiples of G*V).  The warp first
@@ -551,14 +313,6 @@ __device__ __forceinline__ void vec_rows(const LevelArgs& a, int64_t block) {
     }
 }
 
-template <typename T, int V>
-__device__ __forceinline__ Pack<T, V> shfl_xor_pack(const Pack<T, V>& x, int off) {
-    Pack<T, V> r;
-#pragma unroll
-    for (int i = 0; i < V; ++i) r.v[i] = __shfl_xor_sync(kFullMask, x.v[i], off);
-    return r;
-}
-
 // Narrow rows of padded lists, each split over 2^log2s lane groups (default mode only): group
 // j of a row takes quads j, j + 2^log2s, ... and the groups' sums are combined by an
 // xor-shuffle butterfly in a fixed order, so a row waits on ~1/2^log2s of the memory round
@@ -729,22 +483,6 @@ __global__ void __launch_bounds__(kNarrowThreads, MB) level_fused_kernel(LevelAr
 // fresh partial sum per segment, so results are bit-identical to vec_rows; SEG = false adds a
 // row's entries left to right into one sum (default mode only: integer-valued inputs stay
 // exact, real-valued ones differ from the reference by reassociation).
-template <typename T, bool UPONLY>
-__device__ __forceinline__ const T* lean_source(const LevelArgs& a, uint32_t code, bool& ok) {
-    const uint32_t id = code & GRG_B200_ID_MASK;
-    const uint32_t src = (code >> GRG_B200_SRC_SHIFT) & GRG_B200_SRC_MASK;
-    if constexpr (UPONLY) {
-        ok = src == GRG_B200_SRC_STATE;
-        return static_cast<const T*>(a.state) + static_cast<size_t>(id) * static_cast<uint32_t>(a.ld_state);
-    } else {
-        ok = src == GRG_B200_SRC_STATE || src == GRG_B200_SRC_INPUT || (src == GRG_B200_SRC_MISS && a.use_miss);
-        const T* base = src == GRG_B200_SRC_STATE ? static_cast<const T*>(a.state)
-                                                   : (src == GRG_B200_SRC_INPUT ? static_cast<const T*>(a.x) : static_cast<const T*>(a.miss));
-        const uint32_t ld = static_cast<uint32_t>(src == GRG_B200_SRC_STATE ? a.ld_state : (src == GRG_B200_SRC_INPUT ? a.ld_x : a.ld_miss));
-        return base + static_cast<size_t>(id) * ld;
-    }
-}
-
 template <typename T, int V, int INIT, bool SEG, bool UPONLY, int NW = kNarrowWarps>
 __device__ __forceinline__ void lean_rows(const LevelArgs& a, int64_t block) {
     const int warp = threadIdx.x >> 5;
@@ -850,35 +588,6 @@ __device__ __forceinline__ void lean_heavy_rows(const LevelArgs& a, int64_t bloc
             st_pack(state + row * a.ld_state + c, acc);
         }
     }
-}
-
-// 32-byte vector loads and stores (sm_100): one chunk of 4 doubles or 8 floats.
-template <typename T>
-struct Chunk32 {
-    static constexpr int C = 32 / static_cast<int>(sizeof(T));
-    using type = Pack<T, C>;
-};
-
-template <typename T>
-__device__ __forceinline__ typename Chunk32<T>::type ld_chunk(const T* p) {
-    typename Chunk32<T>::type r;
-    if constexpr (std::is_same<T, double>::value) {
-        asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-                     : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p));
-    } else {
-        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]), "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-                     : "l"(p));
-    }
-    return r;
-}
-
-// One chunk lane's CW columns: a 32-byte load when CW fills a chunk, else the shape's vector
-// load (k below a chunk: CW = k, one chunk lane per row).
-template <typename T, int CW>
-__device__ __forceinline__ Pack<T, CW> ld_cols(const T* p) {
-    if constexpr (CW == Chunk32<T>::C) return ld_chunk<T>(p);
-    else return ld_ro<T, CW>(p);
 }
 
 // Narrow rows, entry-parallel (narrow_variant 13, default mode only).  A row's lane group of G
@@ -2151,8 +1860,6 @@ struct Shape {
     int log2g;  // lanes per row = 1 << log2g
 };
 
-bool aligned(const void* p, int bytes) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) % bytes) == 0; }
-
 Shape choose_shape(const grg_b200_traverse_args* a) {
     if (a->dtype == GRG_B200_MIXED) {  // 4 columns per lane (16-byte hi + 8-byte lo loads)
         const int64_t cols = (a->k + 3) / 4;
@@ -2187,41 +1894,41 @@ dim3 grid_for(int64_t rows, int log2g, int threads) {
 }
 
 int validate_common(const grg_b200_traverse_args* a) {
-    if (!a) return fail(GRG_B200_ERR_INVALID, "args is NULL");
+    if (!a) return grg_fail(GRG_B200_ERR_INVALID, "args is NULL");
     if (a->dtype != GRG_B200_F64 && a->dtype != GRG_B200_F32 && a->dtype != GRG_B200_MIXED)
-        return fail(GRG_B200_ERR_INVALID, "unknown dtype %d", a->dtype);
+        return grg_fail(GRG_B200_ERR_INVALID, "unknown dtype %d", a->dtype);
     if (a->dtype == GRG_B200_MIXED) {
         if (a->ld_state % 4 != 0 || !aligned(a->state, 16))
-            return fail(GRG_B200_ERR_INVALID, "mixed state needs ld_state %% 4 == 0 and a 16-byte aligned base");
-        if (a->exact_order) return fail(GRG_B200_ERR_UNSUPPORTED, "mixed storage has no exact-order mode");
+            return grg_fail(GRG_B200_ERR_INVALID, "mixed state needs ld_state %% 4 == 0 and a 16-byte aligned base");
+        if (a->exact_order) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "mixed storage has no exact-order mode");
         if (a->direction == GRG_B200_DOWN) {
             const int64_t need = GRG_B200_MIX_BYTES(a->num_mutations, a->ld_state) * (a->use_miss ? 2 : 1);
             if (!a->mix_scratch || !aligned(a->mix_scratch, 16) || a->mix_scratch_bytes < need)
-                return fail(GRG_B200_ERR_INVALID, "mixed down needs a 16-byte aligned mix_scratch of %lld bytes (got %lld)",
+                return grg_fail(GRG_B200_ERR_INVALID, "mixed down needs a 16-byte aligned mix_scratch of %lld bytes (got %lld)",
                             (long long)need, (long long)a->mix_scratch_bytes);
         }
     }
-    if (a->k < 1) return fail(GRG_B200_ERR_INVALID, "k must be >= 1, got %lld", (long long)a->k);
-    if (a->ld_state < a->k) return fail(GRG_B200_ERR_INVALID, "ld_state %lld < k %lld", (long long)a->ld_state, (long long)a->k);
-    if (!a->state) return fail(GRG_B200_ERR_INVALID, "state is NULL");
+    if (a->k < 1) return grg_fail(GRG_B200_ERR_INVALID, "k must be >= 1, got %lld", (long long)a->k);
+    if (a->ld_state < a->k) return grg_fail(GRG_B200_ERR_INVALID, "ld_state %lld < k %lld", (long long)a->ld_state, (long long)a->k);
+    if (!a->state) return grg_fail(GRG_B200_ERR_INVALID, "state is NULL");
     if (a->num_nodes > (int64_t)GRG_B200_MAX_ID + 1 || a->num_mutations > (int64_t)GRG_B200_MAX_ID + 1)
-        return fail(GRG_B200_ERR_UNSUPPORTED, "node/mutation counts above %u are not supported", GRG_B200_MAX_ID + 1u);
-    if (a->init_mode < 0 || a->init_mode > 3) return fail(GRG_B200_ERR_INVALID, "unknown init_mode %d", a->init_mode);
+        return grg_fail(GRG_B200_ERR_UNSUPPORTED, "node/mutation counts above %u are not supported", GRG_B200_MAX_ID + 1u);
+    if (a->init_mode < 0 || a->init_mode > 3) return grg_fail(GRG_B200_ERR_INVALID, "unknown init_mode %d", a->init_mode);
     if (a->narrow_variant < 0 || a->narrow_variant >= GRG_B200_NARROW_VARIANTS)
-        return fail(GRG_B200_ERR_INVALID, "narrow_variant %d outside [0, %d)", a->narrow_variant, GRG_B200_NARROW_VARIANTS);
-    if (a->heavy_variant < 0 || a->heavy_variant > 3) return fail(GRG_B200_ERR_INVALID, "heavy_variant %d outside [0, 3]", a->heavy_variant);
-    if (a->narrow_split < -1 || a->narrow_split > 3) return fail(GRG_B200_ERR_INVALID, "narrow_split %d outside [-1, 3]", a->narrow_split);
-    if (a->persist_ctas < 0) return fail(GRG_B200_ERR_INVALID, "persist_ctas must be >= 0, got %d", a->persist_ctas);
-    if (a->fuse_entries < 0) return fail(GRG_B200_ERR_INVALID, "fuse_entries must be >= 0, got %lld", (long long)a->fuse_entries);
+        return grg_fail(GRG_B200_ERR_INVALID, "narrow_variant %d outside [0, %d)", a->narrow_variant, GRG_B200_NARROW_VARIANTS);
+    if (a->heavy_variant < 0 || a->heavy_variant > 3) return grg_fail(GRG_B200_ERR_INVALID, "heavy_variant %d outside [0, 3]", a->heavy_variant);
+    if (a->narrow_split < -1 || a->narrow_split > 3) return grg_fail(GRG_B200_ERR_INVALID, "narrow_split %d outside [-1, 3]", a->narrow_split);
+    if (a->persist_ctas < 0) return grg_fail(GRG_B200_ERR_INVALID, "persist_ctas must be >= 0, got %d", a->persist_ctas);
+    if (a->fuse_entries < 0) return grg_fail(GRG_B200_ERR_INVALID, "fuse_entries must be >= 0, got %lld", (long long)a->fuse_entries);
     if (a->schedule != GRG_B200_SCHEDULE_LEVELS && a->schedule != GRG_B200_SCHEDULE_DATAFLOW)
-        return fail(GRG_B200_ERR_INVALID, "unknown schedule %d", a->schedule);
-    if (a->init_mode == GRG_B200_INIT_VECTOR && !a->init_vector) return fail(GRG_B200_ERR_INVALID, "init_vector is NULL");
-    if (a->init_mode == GRG_B200_INIT_XTX && !a->xtx_node) return fail(GRG_B200_ERR_INVALID, "xtx_node is NULL");
+        return grg_fail(GRG_B200_ERR_INVALID, "unknown schedule %d", a->schedule);
+    if (a->init_mode == GRG_B200_INIT_VECTOR && !a->init_vector) return grg_fail(GRG_B200_ERR_INVALID, "init_vector is NULL");
+    if (a->init_mode == GRG_B200_INIT_XTX && !a->xtx_node) return grg_fail(GRG_B200_ERR_INVALID, "xtx_node is NULL");
     if (a->init_mode == GRG_B200_INIT_MATRIX && (!a->init_matrix || !a->node_perm || a->ld_init < a->k))
-        return fail(GRG_B200_ERR_INVALID, "init_matrix/node_perm missing or ld_init < k");
-    if (a->bias_mode < 0 || a->bias_mode > 2) return fail(GRG_B200_ERR_INVALID, "unknown bias_mode %d", a->bias_mode);
-    if (a->bias_mode != GRG_B200_BIAS_NONE && !a->endpoint_bias) return fail(GRG_B200_ERR_INVALID, "endpoint_bias is NULL");
-    if (a->bias_mode == GRG_B200_BIAS_VECTOR && !a->init_vector) return fail(GRG_B200_ERR_INVALID, "init_vector is NULL");
+        return grg_fail(GRG_B200_ERR_INVALID, "init_matrix/node_perm missing or ld_init < k");
+    if (a->bias_mode < 0 || a->bias_mode > 2) return grg_fail(GRG_B200_ERR_INVALID, "unknown bias_mode %d", a->bias_mode);
+    if (a->bias_mode != GRG_B200_BIAS_NONE && !a->endpoint_bias) return grg_fail(GRG_B200_ERR_INVALID, "endpoint_bias is NULL");
+    if (a->bias_mode == GRG_B200_BIAS_VECTOR && !a->init_vector) return grg_fail(GRG_B200_ERR_INVALID, "init_vector is NULL");
     return GRG_B200_OK;
 }
 
@@ -2268,7 +1975,7 @@ int device_sm_count(int* out) {
     static std::atomic<int> cache[64];
     int device = 0;
     GRG_CUDA_TRY(cudaGetDevice(&device));
-    if (device < 0 || device >= 64) return fail(GRG_B200_ERR_UNSUPPORTED, "device ordinal %d above 63", device);
+    if (device < 0 || device >= 64) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "device ordinal %d above 63", device);
     int sms = cache[device].load(std::memory_order_relaxed);
     if (sms <= 0) {
         GRG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -2594,9 +2301,9 @@ int dispatch(const grg_b200_traverse_args* a, const Shape& sh, F&& f) {
 // Checked launch parameters of one non-empty level whose lists are at `blob` (run_level and
 // the fused runs share them).
 int build_level_args(const grg_b200_traverse_args* a, const Shape& sh, const grg_b200_level* L, const void* blob, LevelArgs& out) {
-    if (!blob) return fail(GRG_B200_ERR_INVALID, "level blob is NULL");
+    if (!blob) return grg_fail(GRG_B200_ERR_INVALID, "level blob is NULL");
     if (L->row_begin < 0 || L->row_begin + L->num_rows > a->num_nodes)
-        return fail(GRG_B200_ERR_INVALID, "level rows [%lld, %lld) outside the %lld nodes", (long long)L->row_begin,
+        return grg_fail(GRG_B200_ERR_INVALID, "level rows [%lld, %lld) outside the %lld nodes", (long long)L->row_begin,
                     (long long)(L->row_begin + L->num_rows), (long long)a->num_nodes);
     const char* base = static_cast<const char*>(blob);
     LevelArgs la = level_args(a, sh);
@@ -2606,26 +2313,26 @@ int build_level_args(const grg_b200_traverse_args* a, const Shape& sh, const grg
     la.entries = reinterpret_cast<const uint32_t*>(base + L->off_entries);
     la.heavy_rows = reinterpret_cast<const int32_t*>(base + L->off_heavy);
     la.row_ids = L->off_row_ids >= 0 ? reinterpret_cast<const int32_t*>(base + L->off_row_ids) : nullptr;
-    if (L->list_align != 1 && L->list_align != 4) return fail(GRG_B200_ERR_INVALID, "list_align must be 1 or 4, got %d", L->list_align);
+    if (L->list_align != 1 && L->list_align != 4) return grg_fail(GRG_B200_ERR_INVALID, "list_align must be 1 or 4, got %d", L->list_align);
     if ((a->narrow_variant >= 6 || a->dtype == GRG_B200_MIXED) && L->list_align != 4)
-        return fail(GRG_B200_ERR_INVALID, "narrow_variants 6/7 and mixed storage need padded gather lists (list_align 4)");
-    if (L->list_align == 4 && (L->off_entries % 16) != 0) return fail(GRG_B200_ERR_INVALID, "padded lists must start 16-byte aligned");
+        return grg_fail(GRG_B200_ERR_INVALID, "narrow_variants 6/7 and mixed storage need padded gather lists (list_align 4)");
+    if (L->list_align == 4 && (L->off_entries % 16) != 0) return grg_fail(GRG_B200_ERR_INVALID, "padded lists must start 16-byte aligned");
     la.list_align = L->list_align;
     la.num_heavy = L->num_heavy;
     if (L->short_rows < 0 || L->short_rows > L->num_rows - L->num_heavy)
-        return fail(GRG_B200_ERR_INVALID, "short_rows %lld outside [0, %lld]", (long long)L->short_rows,
+        return grg_fail(GRG_B200_ERR_INVALID, "short_rows %lld outside [0, %lld]", (long long)L->short_rows,
                     (long long)(L->num_rows - L->num_heavy));
     la.short_rows = L->short_rows;
     la.num_slot_buckets = 0;
     if (L->num_slot_buckets < 0 || L->num_slot_buckets > GRG_B200_MAX_SLOT_BUCKETS)
-        return fail(GRG_B200_ERR_INVALID, "num_slot_buckets %d outside [0, %d]", L->num_slot_buckets, GRG_B200_MAX_SLOT_BUCKETS);
+        return grg_fail(GRG_B200_ERR_INVALID, "num_slot_buckets %d outside [0, %d]", L->num_slot_buckets, GRG_B200_MAX_SLOT_BUCKETS);
     if (L->num_slot_buckets > 0) {
-        if (L->list_align != 4 || L->slot_pos[0] != 0) return fail(GRG_B200_ERR_INVALID, "slot table needs padded lists starting at position 0");
+        if (L->list_align != 4 || L->slot_pos[0] != 0) return grg_fail(GRG_B200_ERR_INVALID, "slot table needs padded lists starting at position 0");
         for (int b = 0; b < L->num_slot_buckets; ++b) {
             const int64_t end = b + 1 < L->num_slot_buckets ? L->slot_pos[b + 1] : L->num_rows - L->num_heavy;
             if (L->slot_width[b] < 0 || end < L->slot_pos[b] || L->slot_entry[b] < 0 || (L->slot_entry[b] & 3) ||
                 L->slot_entry[b] + (end - L->slot_pos[b]) * 4 * L->slot_width[b] > L->num_entries)
-                return fail(GRG_B200_ERR_INVALID, "slot bucket %d outside the level's lists", b);
+                return grg_fail(GRG_B200_ERR_INVALID, "slot bucket %d outside the level's lists", b);
             la.slot_pos[b] = L->slot_pos[b];
             la.slot_entry[b] = L->slot_entry[b];
             la.slot_width[b] = L->slot_width[b];
@@ -2653,13 +2360,21 @@ int build_level_args(const grg_b200_traverse_args* a, const Shape& sh, const grg
 
 int run_level(const grg_b200_traverse_args* a, const Shape& sh, const grg_b200_level* L, const void* blob, cudaStream_t s) {
     if (L->num_rows < 0 || L->num_heavy < 0 || L->num_entries < 0)
-        return fail(GRG_B200_ERR_INVALID, "negative level sizes");
+        return grg_fail(GRG_B200_ERR_INVALID, "negative level sizes");
     if (L->num_rows == 0) return GRG_B200_OK;
     LevelArgs la;
     const int rc = build_level_args(a, sh, L, blob, la);
     if (rc) return rc;
     const bool exact = a->exact_order != 0;
     if (a->dtype == GRG_B200_MIXED) return launch_level_mx(la, a->init_mode, a->narrow_variant, s);
+    if ((a->launch_flags & GRG_B200_LAUNCH_WALK) && walk_serves(la, a->init_mode, exact)) {
+        const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
+        for (int i = 0; i < GRG_B200_LONG_CLASSES; ++i)
+            if (L->long_rows[i] < 0 || L->long_rows[i] > L->num_heavy)
+                return grg_fail(GRG_B200_ERR_INVALID, "long_rows[%d] %lld outside [0, %lld]", i, (long long)L->long_rows[i], (long long)L->num_heavy);
+        return a->dtype == GRG_B200_F64 ? launch_walk<double>(la, L->num_entries, L->long_rows, pdl, s)
+                                        : launch_walk<float>(la, L->num_entries, L->long_rows, pdl, s);
+    }
     return dispatch(a, sh, [&](auto t, auto v) {
         return launch_level_typed<decltype(t), decltype(v)::value>(la, a->init_mode, exact, a->narrow_variant, a->heavy_variant,
                                                                    a->persist_ctas, (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0, s);
@@ -2691,7 +2406,7 @@ int launch_run_typed(RunArgs& p, int init_mode, int64_t max_blocks, cudaStream_t
         default: kernel = level_run_kernel<T, V, 3, 5>; break;
     }
     GRG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kNarrowThreads, 0));
-    if (per_sm < 1) return fail(GRG_B200_ERR_UNSUPPORTED, "the fused level run kernel does not fit on an SM");
+    if (per_sm < 1) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "the fused level run kernel does not fit on an SM");
     const int64_t resident = static_cast<int64_t>(sms) * per_sm;
     const int64_t grid = max_blocks < resident ? max_blocks : resident;
     // arrivals and the abort flag restart at zero; a timeout status in sync[2] stays for the host
@@ -2714,7 +2429,7 @@ int launch_run_typed(RunArgs& p, int init_mode, int64_t max_blocks, cudaStream_t
 // Runs levels [first, first + count) (all run_eligible, launch parameters in `las`) as one
 // cooperative launch.
 int launch_run(const grg_b200_traverse_args* a, const Shape& sh, const LevelArgs* las, int count, cudaStream_t s) {
-    if (count < 1 || count > kRunMaxLevels) return fail(GRG_B200_ERR_INVALID, "fused run of %d levels", count);
+    if (count < 1 || count > kRunMaxLevels) return grg_fail(GRG_B200_ERR_INVALID, "fused run of %d levels", count);
     static thread_local RunArgs p;  // about 20 KB: kept off the stack
     std::memset(&p, 0, sizeof(p));
     p.sync = static_cast<int32_t*>(a->dataflow_sync);
@@ -2737,8 +2452,8 @@ int launch_run(const grg_b200_traverse_args* a, const Shape& sh, const LevelArgs
 int seed_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (a->level0_rows <= 0) return GRG_B200_OK;
-    if (!a->input) return fail(GRG_B200_ERR_INVALID, "input is NULL");
-    if (a->by_individual && !a->sample_to_individual) return fail(GRG_B200_ERR_INVALID, "sample_to_individual is NULL");
+    if (!a->input) return grg_fail(GRG_B200_ERR_INVALID, "input is NULL");
+    if (a->by_individual && !a->sample_to_individual) return grg_fail(GRG_B200_ERR_INVALID, "sample_to_individual is NULL");
     LevelArgs la = level_args(a, sh);
     la.row_begin = 0;
     la.num_rows = a->level0_rows;
@@ -2788,8 +2503,8 @@ OutArgs out_args(const grg_b200_traverse_args* a, const Shape& sh) {
 int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (!a->output || !a->sel_mut_ptr || (!a->sel_mut_idx && a->num_mutations > 0))
-        return fail(GRG_B200_ERR_INVALID, "up output needs output and sel_mut");
-    if (a->use_miss && (!a->miss || !a->sel_miss_ptr)) return fail(GRG_B200_ERR_INVALID, "up miss output needs miss and sel_miss");
+        return grg_fail(GRG_B200_ERR_INVALID, "up output needs output and sel_mut");
+    if (a->use_miss && (!a->miss || !a->sel_miss_ptr)) return grg_fail(GRG_B200_ERR_INVALID, "up miss output needs miss and sel_miss");
     if (a->num_mutations == 0) return GRG_B200_OK;
     OutArgs o = out_args(a, sh);
     o.rows = a->num_mutations;
@@ -2832,10 +2547,10 @@ int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_
 
 int output_down_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
-    if (!a->output) return fail(GRG_B200_ERR_INVALID, "output is NULL");
+    if (!a->output) return grg_fail(GRG_B200_ERR_INVALID, "output is NULL");
     OutArgs o = out_args(a, sh);
     if (a->by_individual) {
-        if (!a->ind_ptr || !a->ind_samples) return fail(GRG_B200_ERR_INVALID, "by_individual needs ind_ptr/ind_samples");
+        if (!a->ind_ptr || !a->ind_samples) return grg_fail(GRG_B200_ERR_INVALID, "by_individual needs ind_ptr/ind_samples");
         o.rows = a->num_individuals;
         o.ptr = a->ind_ptr;
         o.idx = a->ind_samples;
@@ -2863,7 +2578,7 @@ int output_down_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStrea
 
 int emit_all_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
-    if (!a->output || !a->inv_node_perm) return fail(GRG_B200_ERR_INVALID, "emit_all_nodes needs output and inv_node_perm");
+    if (!a->output || !a->inv_node_perm) return grg_fail(GRG_B200_ERR_INVALID, "emit_all_nodes needs output and inv_node_perm");
     OutArgs o = out_args(a, sh);
     o.rows = a->num_nodes;
     o.idx = a->inv_node_perm;
@@ -2925,10 +2640,10 @@ int run_dataflow(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t 
     for (int i = 0; i < a->num_levels; ++i) {
         const grg_b200_level& L = a->levels[i];
         const char* base = static_cast<const char*>(L.blob);
-        if (L.num_rows > 0 && !base) return fail(GRG_B200_ERR_INVALID, "level blob is NULL");
+        if (L.num_rows > 0 && !base) return grg_fail(GRG_B200_ERR_INVALID, "level blob is NULL");
         if (L.row_begin < 0 || L.row_begin + L.num_rows > a->num_nodes)
-            return fail(GRG_B200_ERR_INVALID, "level rows outside the %lld nodes", (long long)a->num_nodes);
-        if (L.list_align == 4 && (L.off_entries % 16) != 0) return fail(GRG_B200_ERR_INVALID, "padded lists must start 16-byte aligned");
+            return grg_fail(GRG_B200_ERR_INVALID, "level rows outside the %lld nodes", (long long)a->num_nodes);
+        if (L.list_align == 4 && (L.off_entries % 16) != 0) return grg_fail(GRG_B200_ERR_INVALID, "padded lists must start 16-byte aligned");
         DfLevel& d = p.lv[i];
         d.row_ptr = reinterpret_cast<const int32_t*>(base + L.off_row_ptr);
         d.codes = reinterpret_cast<const uint4*>(base + L.off_entries);
@@ -2944,7 +2659,7 @@ int run_dataflow(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t 
             fill_end = L.row_begin + L.num_rows > fill_end ? L.row_begin + L.num_rows : fill_end;
         }
     }
-    if (tasks >= INT32_MAX) return fail(GRG_B200_ERR_UNSUPPORTED, "dataflow schedule: too many tasks");
+    if (tasks >= INT32_MAX) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "dataflow schedule: too many tasks");
     p.task_begin[a->num_levels] = static_cast<int32_t>(tasks);
     p.total_tasks = static_cast<int32_t>(tasks);
     GRG_CUDA_TRY(cudaMemsetAsync(a->dataflow_sync, 0, 4 * sizeof(int32_t), s));
@@ -3069,21 +2784,21 @@ extern "C" {
 int grg_b200_abi_version(void) { return GRG_B200_ABI_VERSION; }
 
 int grg_b200_rowop(const grg_b200_rowop_args* a, void* stream_handle) {
-    if (!a) return fail(GRG_B200_ERR_INVALID, "args is NULL");
+    if (!a) return grg_fail(GRG_B200_ERR_INVALID, "args is NULL");
     if (a->rows < 0 || a->k < 1 || a->ld < a->k)
-        return fail(GRG_B200_ERR_INVALID, "rowop needs rows >= 0, k >= 1 and ld >= k (got %lld, %lld, %lld)",
+        return grg_fail(GRG_B200_ERR_INVALID, "rowop needs rows >= 0, k >= 1 and ld >= k (got %lld, %lld, %lld)",
                     (long long)a->rows, (long long)a->k, (long long)a->ld);
-    if (!a->src || !a->dst) return fail(GRG_B200_ERR_INVALID, "rowop src/dst is NULL");
-    if (a->miss_in && !a->miss_scale) return fail(GRG_B200_ERR_INVALID, "rowop miss_in needs miss_scale");
-    if (a->miss_out && !a->miss_out_scale) return fail(GRG_B200_ERR_INVALID, "rowop miss_out needs miss_out_scale");
-    if (a->col_sums && (!a->partials || !a->sums)) return fail(GRG_B200_ERR_INVALID, "rowop col_sums needs partials and sums");
+    if (!a->src || !a->dst) return grg_fail(GRG_B200_ERR_INVALID, "rowop src/dst is NULL");
+    if (a->miss_in && !a->miss_scale) return grg_fail(GRG_B200_ERR_INVALID, "rowop miss_in needs miss_scale");
+    if (a->miss_out && !a->miss_out_scale) return grg_fail(GRG_B200_ERR_INVALID, "rowop miss_out needs miss_out_scale");
+    if (a->col_sums && (!a->partials || !a->sums)) return grg_fail(GRG_B200_ERR_INVALID, "rowop col_sums needs partials and sums");
     if (a->rows == 0) return GRG_B200_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream_handle);
     int log2kt = 0;
     while ((int64_t{1} << log2kt) < a->k && log2kt < 8) ++log2kt;
     const int64_t blocks = GRG_B200_ROWOP_BLOCKS(a->rows);
     const int64_t rows_per_block = (a->rows + blocks - 1) / blocks;
-    if (a->k > 0x7fffffff) return fail(GRG_B200_ERR_UNSUPPORTED, "rowop: k = %lld is too large", (long long)a->k);
+    if (a->k > 0x7fffffff) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "rowop: k = %lld is too large", (long long)a->k);
     rowop_kernel<<<dim3(static_cast<unsigned>(blocks)), kRowopThreads, 0, s>>>(*a, log2kt, rows_per_block);
     GRG_LAUNCH_CHECK("rowop_kernel");
     if (a->col_sums) {
@@ -3105,7 +2820,7 @@ size_t grg_b200_last_error(char* buf, size_t buf_size) {
 }
 
 int grg_b200_ring_create(int device, int num_slots, grg_b200_ring** out) {
-    if (!out || num_slots < 1) return fail(GRG_B200_ERR_INVALID, "ring needs num_slots >= 1 and an out pointer");
+    if (!out || num_slots < 1) return grg_fail(GRG_B200_ERR_INVALID, "ring needs num_slots >= 1 and an out pointer");
     *out = nullptr;
     int prev = 0;
     GRG_CUDA_TRY(cudaGetDevice(&prev));
@@ -3125,7 +2840,7 @@ int grg_b200_ring_create(int device, int num_slots, grg_b200_ring** out) {
     cudaSetDevice(prev);
     if (e != cudaSuccess) {
         grg_b200_ring_destroy(r);
-        return fail(GRG_B200_ERR_CUDA, "ring creation failed: %s", cudaGetErrorString(e));
+        return grg_fail(GRG_B200_ERR_CUDA, "ring creation failed: %s", cudaGetErrorString(e));
     }
     *out = r;
     return GRG_B200_OK;
@@ -3160,7 +2875,7 @@ int grg_b200_seed_up(const grg_b200_traverse_args* a, void* stream) {
 int grg_b200_run_level(const grg_b200_traverse_args* a, const grg_b200_level* level, void* stream) {
     int rc = validate_common(a);
     if (rc) return rc;
-    if (!level) return fail(GRG_B200_ERR_INVALID, "level is NULL");
+    if (!level) return grg_fail(GRG_B200_ERR_INVALID, "level is NULL");
     return run_level(a, choose_shape(a), level, level->blob, static_cast<cudaStream_t>(stream));
 }
 
@@ -3185,9 +2900,9 @@ int grg_b200_emit_all(const grg_b200_traverse_args* a, void* stream) {
 int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
     int rc = validate_common(a);
     if (rc) return rc;
-    if (a->num_levels < 0 || (a->num_levels > 0 && !a->levels)) return fail(GRG_B200_ERR_INVALID, "levels missing");
-    if (a->direction == GRG_B200_DOWN && !a->input && a->num_mutations > 0) return fail(GRG_B200_ERR_INVALID, "input is NULL");
-    if (a->direction == GRG_B200_DOWN && a->use_miss && !a->miss) return fail(GRG_B200_ERR_INVALID, "miss input is NULL");
+    if (a->num_levels < 0 || (a->num_levels > 0 && !a->levels)) return grg_fail(GRG_B200_ERR_INVALID, "levels missing");
+    if (a->direction == GRG_B200_DOWN && !a->input && a->num_mutations > 0) return grg_fail(GRG_B200_ERR_INVALID, "input is NULL");
+    if (a->direction == GRG_B200_DOWN && a->use_miss && !a->miss) return grg_fail(GRG_B200_ERR_INVALID, "miss input is NULL");
     cudaStream_t s = static_cast<cudaStream_t>(stream_handle);
     const Shape sh = choose_shape(a);
 
@@ -3197,9 +2912,9 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
         if (L.ring_slot >= 0) {
             any_streamed = true;
             if (!a->ring || L.ring_slot >= a->num_slots || L.ring_slot >= a->ring->num_slots || !a->slot_buffers || !a->slot_bytes)
-                return fail(GRG_B200_ERR_INVALID, "level %d is streamed through slot %d but the ring is missing or too small", i, L.ring_slot);
+                return grg_fail(GRG_B200_ERR_INVALID, "level %d is streamed through slot %d but the ring is missing or too small", i, L.ring_slot);
             if (L.blob_bytes > a->slot_bytes[L.ring_slot])
-                return fail(GRG_B200_ERR_INVALID, "level %d needs %lld bytes, slot %d has %lld", i, (long long)L.blob_bytes,
+                return grg_fail(GRG_B200_ERR_INVALID, "level %d needs %lld bytes, slot %d has %lld", i, (long long)L.blob_bytes,
                             L.ring_slot, (long long)a->slot_bytes[L.ring_slot]);
         }
     }
@@ -3228,7 +2943,7 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
     // caller's earlier work (and join a CUDA graph capture in progress).
     bool used[256] = {false};
     if (any_streamed) {
-        if (a->ring->num_slots > 256) return fail(GRG_B200_ERR_UNSUPPORTED, "at most 256 ring slots");
+        if (a->ring->num_slots > 256) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "at most 256 ring slots");
         GRG_CUDA_TRY(cudaEventRecord(a->ring->fork, s));
         GRG_CUDA_TRY(cudaStreamWaitEvent(a->ring->copy, a->ring->fork, 0));
     }
@@ -3322,14 +3037,14 @@ void* current_context() {
 int static_state_address(void** out) {
     int device = 0;
     GRG_CUDA_TRY(cudaGetDevice(&device));
-    if (device < 0 || device >= kMaxDevices) return fail(GRG_B200_ERR_UNSUPPORTED, "device ordinal %d above %d", device, kMaxDevices);
+    if (device < 0 || device >= kMaxDevices) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "device ordinal %d above %d", device, kMaxDevices);
     void* ctx = current_context();  // nullptr before the runtime has made a context current
     std::lock_guard<std::mutex> lock(g_static_mutex);
     if (!g_static_ptr[device] || !ctx || g_static_ctx[device] != ctx) {
         void* ptr = nullptr;
         const cudaError_t err = cudaGetSymbolAddress(&ptr, g_static_state);  // makes the context current
         if (err != cudaSuccess || !ptr)
-            return fail(GRG_B200_ERR_CUDA, "cudaGetSymbolAddress(g_static_state) on device %d failed: %s", device,
+            return grg_fail(GRG_B200_ERR_CUDA, "cudaGetSymbolAddress(g_static_state) on device %d failed: %s", device,
                         cudaGetErrorString(err));
         g_static_ptr[device] = ptr;
         g_static_ctx[device] = current_context();
@@ -3340,18 +3055,18 @@ int static_state_address(void** out) {
 }  // namespace
 
 int grg_b200_traverse_static(const grg_b200_traverse_args* a, void* stream_handle) {
-    if (!a) return fail(GRG_B200_ERR_INVALID, "args is NULL");
-    if (a->k < 1) return fail(GRG_B200_ERR_INVALID, "k must be >= 1, got %lld", (long long)a->k);
-    if (a->dtype == GRG_B200_MIXED) return fail(GRG_B200_ERR_UNSUPPORTED, "grg_b200_traverse_static serves the FP64 and FP32 dtypes only");
+    if (!a) return grg_fail(GRG_B200_ERR_INVALID, "args is NULL");
+    if (a->k < 1) return grg_fail(GRG_B200_ERR_INVALID, "k must be >= 1, got %lld", (long long)a->k);
+    if (a->dtype == GRG_B200_MIXED) return grg_fail(GRG_B200_ERR_UNSUPPORTED, "grg_b200_traverse_static serves the FP64 and FP32 dtypes only");
     const int64_t esize = a->dtype == GRG_B200_F64 ? 8 : 4;
     if (a->num_nodes < 0 || a->num_nodes > (int64_t)GRG_B200_STATIC_STATE_BYTES / esize / a->k)
-        return fail(GRG_B200_ERR_UNSUPPORTED,
+        return grg_fail(GRG_B200_ERR_UNSUPPORTED,
                     "grg_b200_traverse_static holds at most %lld bytes of node state; %lld nodes x k=%lld need %lld",
                     (long long)GRG_B200_STATIC_STATE_BYTES, (long long)a->num_nodes, (long long)a->k,
                     (long long)(a->num_nodes * a->k * esize));
     for (int i = 0; a->levels && i < a->num_levels; ++i)
         if (a->levels[i].ring_slot >= 0)
-            return fail(GRG_B200_ERR_UNSUPPORTED, "grg_b200_traverse_static needs every level resident (level %d is streamed)", i);
+            return grg_fail(GRG_B200_ERR_UNSUPPORTED, "grg_b200_traverse_static needs every level resident (level %d is streamed)", i);
     void* state = nullptr;
     const int rc = static_state_address(&state);
     if (rc) return rc;

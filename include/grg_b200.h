@@ -55,7 +55,7 @@
 extern "C" {
 #endif
 
-#define GRG_B200_ABI_VERSION 14
+#define GRG_B200_ABI_VERSION 15
 
 typedef enum grg_b200_status {
     GRG_B200_OK = 0,
@@ -111,7 +111,8 @@ typedef enum grg_b200_bias {
  * positions (split across a warp or a CTA per row, heavy_variant); narrow kernels cover the
  * first num_rows - num_heavy:
  *   int32  row_ptr[num_rows + 1]     entry offsets of each processing position
- *   int32  heavy_rows[num_heavy]     the heavy positions (num_rows - num_heavy, ...)
+ *   int32  heavy_rows[num_heavy]     the heavy positions (num_rows - num_heavy, ...), the rows
+ *                                    that long_rows counts first
  *   int32  row_ids[num_rows]         optional processing position -> level-local row
  *   uint32 entries[num_entries]
  * list_align = 4: every position's list starts at a multiple of 4 entries and holds a
@@ -124,6 +125,10 @@ typedef enum grg_b200_bias {
  * same number of 4-entry quads, so a kernel computes a row's list from its position
  * (slot_entry[b] + (p - slot_pos[b]) * 4 * slot_width[b]) instead of loading row_ptr. */
 #define GRG_B200_MAX_SLOT_BUCKETS 8
+
+/* Very long rows: class i holds the rows of more than GRG_B200_LONG_ROW << i entries. */
+#define GRG_B200_LONG_ROW 512
+#define GRG_B200_LONG_CLASSES 8
 
 typedef struct grg_b200_level {
     int64_t row_begin;
@@ -148,6 +153,10 @@ typedef struct grg_b200_level {
                            them with one entry slot, twice the rows per CTA.  A speed hint:
                            longer lists there still sum correctly.  0 <= short_rows <=
                            num_rows - num_heavy; 0 for none. */
+    int64_t long_rows[GRG_B200_LONG_CLASSES]; /* long_rows[i]: how many of the heavy rows hold more
+                           than GRG_B200_LONG_ROW << i entries; heavy_rows lists them first, longest
+                           class first, so they are its first long_rows[i] members.  0 for all when
+                           heavy_rows is in another order. */
 } grg_b200_level;
 
 typedef struct grg_b200_ring grg_b200_ring; /* opaque: copy stream + per-slot events */
@@ -266,6 +275,11 @@ typedef struct grg_b200_traverse_args {
  * level lists until the hardware reports that kernel complete, and so overlaps the launch
  * gap.  Ignored when any level is streamed. */
 #define GRG_B200_LAUNCH_PDL 1
+
+/* Let the library choose the row walk of every level from k, the buffers and the level's sizes
+ * (default mode, FP64/FP32, padded lists, no error word, no init inside the traversal; other
+ * launches use narrow_variant and heavy_variant). */
+#define GRG_B200_LAUNCH_WALK 2
 
 /*
  * GRG_B200_SCHEDULE_LEVELS: one launch per level (each level waits for the previous one).
