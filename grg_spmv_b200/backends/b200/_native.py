@@ -15,7 +15,7 @@ import threading
 PACKAGE_DIR = Path(__file__).resolve().parents[2]
 REPO_DIR = PACKAGE_DIR.parent
 LIB_PATH = PACKAGE_DIR / "libgrg_b200.so"
-SOURCES = (PACKAGE_DIR / "csrc" / "grg_b200.cu", PACKAGE_DIR / "csrc" / "level_walk.cu")
+SOURCES = tuple(PACKAGE_DIR / "csrc" / name for name in ("grg_b200.cu", "level_walk.cu", "level_walk_mixed.cu"))
 OBJECT_DIR = PACKAGE_DIR / "_build"
 HEADER_DIR = REPO_DIR / "include"
 ABI_VERSION = 15
@@ -48,7 +48,7 @@ def mix_plane(nbytes: int) -> int:
 
 
 def mix_bytes(rows: int, ld: int) -> int:
-    """GRG_B200_MIX_BYTES: one mixed buffer (float hi plane, then int16 lo plane)."""
+    """GRG_B200_MIX_BYTES: one mixed buffer (uint32 hi plane, then uint16 lo plane)."""
     return mix_plane(int(rows) * int(ld) * 4) + mix_plane(int(rows) * int(ld) * 2)
 
 

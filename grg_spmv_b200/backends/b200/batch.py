@@ -14,7 +14,7 @@ latency-bound gather, so one such walk leaves most of a B200 idle.  A batch inst
   traversals overlap on the GPU; one replay runs the whole batch.
 
 With ``precision="mixed"`` the tiles keep their node state in the 6-byte mixed form of
-``grg_b200.h`` (FP32 value + 16-bit correction, FP64 sums); inputs and outputs stay FP64.
+``grg_b200.h`` (FP32 value + 16 more mantissa bits, FP64 sums); inputs and outputs stay FP64.
 
 Every buffer of the batch is allocated when it is prepared and freed by ``close()``; calls
 allocate nothing.  Levels must be resident (a streamed level would share the runtime's one

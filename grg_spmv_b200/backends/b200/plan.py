@@ -435,8 +435,8 @@ def plan_b200_layout(
 
     ``precision="plain"`` computes and stores in ``dtype``.  ``precision="mixed"`` (``dtype``
     must be float64: inputs and outputs stay FP64) keeps the node state in 6 bytes per value,
-    an FP32 value plus a 16-bit correction (relative rounding <= 2^-39 per node, integers below
-    2^39 exact), with FP64 accumulation; it needs padded lists and the default (not
+    an FP32 value plus 16 further mantissa bits (relative rounding <= 2^-40 per node, integers up
+    to 2^40 exact), with FP64 accumulation; it needs padded lists and the default (not
     exact-order) heavy-row mode.
 
     ``emit_all_nodes=False`` leaves out the all-node output buffer (``max_nodes x max_k``
@@ -484,7 +484,7 @@ def _check_precision(precision: str, dtype, pair: B200PlanPair) -> None:
 
 
 def mixed_state_bytes(num_nodes: int, max_k: int) -> int:
-    """Node state of mixed precision: float hi plane + int16 lo plane, ld = k rounded up to 4."""
+    """Node state of mixed precision: uint32 hi plane + uint16 lo plane, ld = k rounded up to 4."""
     ld = (int(max_k) + 3) // 4 * 4
     return _plane(num_nodes * ld * 4) + _plane(num_nodes * ld * 2)
 

@@ -205,7 +205,7 @@ class B200Runtime:
             with torch.cuda.device(self.device):
                 self._caller_stream = torch.cuda.get_stream_from_external(self.stream_ptr, device=self.device)
                 self.stream = self._caller_stream
-                if lay.precision == "mixed":  # float hi plane + int16 lo plane (grg_b200.h GRG_B200_MIXED)
+                if lay.precision == "mixed":  # uint32 hi plane + uint16 lo plane (grg_b200.h GRG_B200_MIXED)
                     self._state = torch.zeros(nat.mix_bytes(lay.max_num_nodes, nat.mix_ld(max_k)), device=self.device,
                                               dtype=torch.uint8)
                     if lay.mix_scratch_bytes:

@@ -96,8 +96,10 @@ class LevelGather:
     def long_rows(self) -> list[int]:
         """How many heavy rows hold more than ``LONG_ROW << i`` entries: the first so many of
         ``heavy_rows``, which kernels may split further than the others."""
-        lengths = self.row_ptr[self.heavy_rows + 1].astype(np.int64) - self.row_ptr[self.heavy_rows]
-        return [int((lengths > (nat.LONG_ROW << i)).sum()) for i in range(nat.LONG_CLASSES)]
+        if self.heavy_rows.size == 0:
+            return [0] * nat.LONG_CLASSES
+        lengths = np.sort(self.row_ptr[self.heavy_rows + 1] - self.row_ptr[self.heavy_rows])
+        return (lengths.size - np.searchsorted(lengths, _LONG, side="right")).tolist()
 
     def layout(self) -> tuple[int, int, int, int, int]:
         return blob_layout(self.num_rows, self.heavy_rows.size, self.entries.size, self.row_ids is not None)
@@ -153,7 +155,9 @@ def _heavy_rows(row_ptr: np.ndarray, num_rows: int, num_heavy: int) -> np.ndarra
     """The heavy positions (the suffix), those in the longest classes of ``long_rows`` first and
     in processing order inside a class."""
     first = num_rows - num_heavy
-    lengths = np.diff(row_ptr[first:].astype(np.int64))
+    lengths = np.diff(row_ptr[first:])
+    if num_heavy == 0 or int(lengths.max()) <= nat.LONG_ROW:
+        return np.arange(first, num_rows, dtype=np.int32)
     long_class = np.searchsorted(_LONG, lengths, side="left")  # lengths above LONG_ROW << i, counted over i
     return (first + np.argsort(-long_class, kind="stable")).astype(np.int32)
 

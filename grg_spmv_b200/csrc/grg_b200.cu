@@ -35,6 +35,7 @@
 
 #include "level_common.cuh"
 #include "level_walk.h"
+#include "mixed.cuh"
 
 namespace {
 
@@ -983,337 +984,12 @@ __global__ void __launch_bounds__(kNarrowThreads, MB) level_run_kernel(const __g
 }
 
 // ---------------------------------------------------------------------------------------
-// Mixed storage (dtype GRG_B200_MIXED)
-//
-// A value v is stored in 6 bytes as hi = v rounded to nearest FP32 plus a 16-bit signed
-// correction lo, so that v ~= hi + lo * 2^(e(hi) - 38), where e(hi) is hi's unbiased exponent
-// (FP32 subnormals use the smallest normal exponent).  |v - hi| is at most half an FP32 ulp,
-// 2^(e - 24), so |lo| <= 2^14 always fits; the stored value is within 2^-39 of v relative to
-// |hi| and integers below 2^39 are exact.  Decoding is exact in FP64 (24 + 15 bits fit in 53),
-// every sum is accumulated in FP64 registers and rounded back to 6 bytes once per node.  A buffer of R rows and ld
-// columns (ld % 4 == 0) is two planes: float hi[R * ld] followed by int16 lo[R * ld].
+// Mixed storage (dtype GRG_B200_MIXED, mixed.cuh): inputs in and out.  A buffer of R rows and ld
+// columns (ld % 4 == 0) is two planes: uint32 hi[R * ld] followed by uint16 lo[R * ld].
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t mx_exp_field(float hi) {
-    const uint32_t e = (__float_as_uint(hi) >> 23) & 0xffu;
-    return e == 0u ? 1u : e;
-}
-
-// 2^(e - 38) for the biased exponent field E = e + 127: 2^(E - 165) as a double.
-__device__ __forceinline__ double mx_unit(float hi) {
-    return __longlong_as_double(static_cast<long long>(mx_exp_field(hi) + (1023u - 165u)) << 52);
-}
-
-__device__ __forceinline__ double mx_inv_unit(float hi) {
-    return __longlong_as_double(static_cast<long long>((1023u + 165u) - mx_exp_field(hi)) << 52);
-}
-
-__device__ __forceinline__ double mx_decode(float hi, short lo) {
-    return static_cast<double>(hi) + static_cast<double>(lo) * mx_unit(hi);
-}
-
-__device__ __forceinline__ void mx_encode(double v, float& hi, short& lo) {
-    hi = __double2float_rn(v);
-    if (!isfinite(hi)) {
-        lo = 0;
-        return;
-    }
-    const double r = v - static_cast<double>(hi);  // exact
-    lo = static_cast<short>(__double2int_rn(r * mx_inv_unit(hi)));  // |lo| <= 2^14
-}
-
-struct Quad {
-    double v[4];
-};
-
-__device__ __forceinline__ Quad zero_quad() { return Quad{{0.0, 0.0, 0.0, 0.0}}; }
-
-__device__ __forceinline__ void add_quad(Quad& a, const Quad& b) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a.v[i] = a.v[i] + b.v[i];
-}
-
-// Four encoded columns [c, c + 4) as loaded (16-byte hi load + 8-byte lo load).
-struct RawQuad {
-    float4 h;
-    short4 l;
-};
-
-__device__ __forceinline__ RawQuad mx_load_raw(const float* hi_row, const short* lo_row) {
-    return RawQuad{__ldg(reinterpret_cast<const float4*>(hi_row)), __ldg(reinterpret_cast<const short4*>(lo_row))};
-}
-
-__device__ __forceinline__ void add_raw(Quad& a, const RawQuad& r) {
-    a.v[0] = a.v[0] + mx_decode(r.h.x, r.l.x);
-    a.v[1] = a.v[1] + mx_decode(r.h.y, r.l.y);
-    a.v[2] = a.v[2] + mx_decode(r.h.z, r.l.z);
-    a.v[3] = a.v[3] + mx_decode(r.h.w, r.l.w);
-}
-
-__device__ __forceinline__ Quad mx_load(const float* hi_row, const short* lo_row) {
-    Quad q = zero_quad();
-    add_raw(q, mx_load_raw(hi_row, lo_row));
-    return q;
-}
-
-__device__ __forceinline__ void mx_store(float* hi_row, short* lo_row, const Quad& q) {
-    float4 h;
-    short4 l;
-    mx_encode(q.v[0], h.x, l.x);
-    mx_encode(q.v[1], h.y, l.y);
-    mx_encode(q.v[2], h.z, l.z);
-    mx_encode(q.v[3], h.w, l.w);
-    *reinterpret_cast<float4*>(hi_row) = h;
-    *reinterpret_cast<short4*>(lo_row) = l;
-}
-
-// Columns [c, c + 4) of an FP64 row with columns >= k read as zero.
-__device__ __forceinline__ Quad f64_load_guarded(const double* row, int64_t c, int64_t k) {
-    Quad q;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) q.v[i] = c + i < k ? __ldg(row + c + i) : 0.0;
-    return q;
-}
-
-__device__ __forceinline__ void f64_store_guarded(double* row, int64_t c, int64_t k, const Quad& q) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        if (c + i < k) row[c + i] = q.v[i];
-}
-
-template <int INIT>
-__device__ __forceinline__ Quad mx_init(const LevelArgs& a, int64_t row, int64_t c) {
-    if constexpr (INIT == GRG_B200_INIT_VECTOR) {
-        return f64_load_guarded(static_cast<const double*>(a.init_vector), c, a.k);
-    } else if constexpr (INIT == GRG_B200_INIT_XTX) {
-        const double x = __ldg(static_cast<const double*>(a.xtx_node) + row);
-        return Quad{{x, x, x, x}};
-    } else if constexpr (INIT == GRG_B200_INIT_MATRIX) {
-        const int64_t orig = __ldg(a.node_perm + row);
-        if (a.err && (orig < 0 || orig >= a.lim_state)) {
-            report(a.err, kErrPerm);
-            return zero_quad();
-        }
-        return f64_load_guarded(static_cast<const double*>(a.init_matrix) + orig * a.ld_init, c, a.k);
-    } else {
-        return zero_quad();
-    }
-}
-
-// Encoded row named by a coded entry (hi and lo row starts); false when the entry is skipped.
-__device__ __forceinline__ bool mx_entry(const LevelArgs& a, uint32_t code, const float*& hi, const short*& lo) {
-    const uint32_t src = (code >> GRG_B200_SRC_SHIFT) & GRG_B200_SRC_MASK;
-    const int64_t id = code & GRG_B200_ID_MASK;
-    int64_t off;
-    if (src == GRG_B200_SRC_STATE) {
-        if (a.err && id >= a.lim_state) {
-            report(a.err, kErrStateId);
-            return false;
-        }
-        off = id * a.ld_state;
-        hi = static_cast<const float*>(a.state) + off;
-        lo = static_cast<const short*>(a.state_lo) + off;
-        return true;
-    }
-    if (src == GRG_B200_SRC_INPUT) {
-        if (a.err && id >= a.lim_x) {
-            report(a.err, kErrInputId);
-            return false;
-        }
-        off = id * a.ld_x;
-        hi = static_cast<const float*>(a.x) + off;
-        lo = static_cast<const short*>(a.x_lo) + off;
-        return true;
-    }
-    if (src != GRG_B200_SRC_MISS || !a.use_miss) return false;
-    if (a.err && id >= a.lim_miss) {
-        report(a.err, kErrMissId);
-        return false;
-    }
-    off = id * a.ld_miss;
-    hi = static_cast<const float*>(a.miss) + off;
-    lo = static_cast<const short*>(a.miss_lo) + off;
-    return true;
-}
-
-// Generic VM-column pieces of the mixed level kernels (VM = 4: 16-byte hi + 8-byte lo loads;
-// VM = 2: 8-byte hi + 4-byte lo loads, half the registers per lane, twice the lanes per row).
-template <int VM>
-struct MxRaw;
-template <>
-struct MxRaw<4> {
-    float4 h;
-    short4 l;
-};
-template <>
-struct MxRaw<2> {
-    float2 h;
-    short2 l;
-};
-
-template <int VM>
-__device__ __forceinline__ MxRaw<VM> mx_ld(const float* hi, const short* lo) {
-    if constexpr (VM == 4)
-        return MxRaw<4>{__ldg(reinterpret_cast<const float4*>(hi)), __ldg(reinterpret_cast<const short4*>(lo))};
-    else
-        return MxRaw<2>{__ldg(reinterpret_cast<const float2*>(hi)), __ldg(reinterpret_cast<const short2*>(lo))};
-}
-
-template <int VM>
-__device__ __forceinline__ MxRaw<VM> mx_zero() {
-    if constexpr (VM == 4) return MxRaw<4>{make_float4(0.f, 0.f, 0.f, 0.f), make_short4(0, 0, 0, 0)};
-    else return MxRaw<2>{make_float2(0.f, 0.f), make_short2(0, 0)};
-}
-
-template <int VM>
-__device__ __forceinline__ void mx_add(Pack<double, VM>& a, const MxRaw<VM>& r) {
-    a.v[0] = a.v[0] + mx_decode(r.h.x, r.l.x);
-    a.v[1] = a.v[1] + mx_decode(r.h.y, r.l.y);
-    if constexpr (VM == 4) {
-        a.v[2] = a.v[2] + mx_decode(r.h.z, r.l.z);
-        a.v[3] = a.v[3] + mx_decode(r.h.w, r.l.w);
-    }
-}
-
-template <int VM>
-__device__ __forceinline__ void mx_st(float* hi, short* lo, const Pack<double, VM>& v) {
-    if constexpr (VM == 4) {
-        mx_store(hi, lo, Quad{{v.v[0], v.v[1], v.v[2], v.v[3]}});
-    } else {
-        float2 h;
-        short2 l;
-        mx_encode(v.v[0], h.x, l.x);
-        mx_encode(v.v[1], h.y, l.y);
-        *reinterpret_cast<float2*>(hi) = h;
-        *reinterpret_cast<short2*>(lo) = l;
-    }
-}
-
-template <int VM>
-__device__ __forceinline__ Pack<double, VM> f64_ld_guarded(const double* row, int64_t c, int64_t k) {
-    Pack<double, VM> q;
-#pragma unroll
-    for (int i = 0; i < VM; ++i) q.v[i] = c + i < k ? __ldg(row + c + i) : 0.0;
-    return q;
-}
-
-template <int INIT, int VM>
-__device__ __forceinline__ Pack<double, VM> mx_init_v(const LevelArgs& a, int64_t row, int64_t c) {
-    if constexpr (INIT == GRG_B200_INIT_VECTOR) {
-        return f64_ld_guarded<VM>(static_cast<const double*>(a.init_vector), c, a.k);
-    } else if constexpr (INIT == GRG_B200_INIT_XTX) {
-        return splat<double, VM>(__ldg(static_cast<const double*>(a.xtx_node) + row));
-    } else if constexpr (INIT == GRG_B200_INIT_MATRIX) {
-        const int64_t orig = __ldg(a.node_perm + row);
-        if (a.err && (orig < 0 || orig >= a.lim_state)) {
-            report(a.err, kErrPerm);
-            return zero_pack<double, VM>();
-        }
-        return f64_ld_guarded<VM>(static_cast<const double*>(a.init_matrix) + orig * a.ld_init, c, a.k);
-    } else {
-        return zero_pack<double, VM>();
-    }
-}
-
-// Narrow rows of padded lists in mixed storage: the ownership and code prefetch of
-// level_vec_kernel with VM columns per lane; adds in list order, segment by segment.
-template <int INIT, int VM>
-__global__ void __launch_bounds__(kNarrowThreads, VM == 4 ? 3 : 5) level_mx_kernel(LevelArgs a) {
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const int64_t narrow = a.num_rows - a.num_heavy;
-    const int64_t pos = ((static_cast<int64_t>(blockIdx.x) * kNarrowWarps + warp) << (5 - a.log2g)) + (lane >> a.log2g);
-    if (pos >= narrow) return;
-    const int32_t e0 = __ldg(a.row_ptr + pos);
-    const int32_t e1 = __ldg(a.row_ptr + pos + 1);
-    const int glane = lane & ((1 << a.log2g) - 1);
-    const int64_t row = level_row(a, pos);
-    const uint4* codes4 = reinterpret_cast<const uint4*>(a.entries);
-    const uint32_t null_code = GRG_B200_SRC_NULL << GRG_B200_SRC_SHIFT;
-    const uint4 null4 = make_uint4(null_code, null_code, null_code, null_code);
-    const int64_t step = static_cast<int64_t>(VM) << a.log2g;
-    for (int64_t c = static_cast<int64_t>(glane) * VM; c < a.k; c += step) {
-        Pack<double, VM> acc = mx_init_v<INIT, VM>(a, row, c);
-        Pack<double, VM> seg = zero_pack<double, VM>();
-        const int32_t q1 = e1 >> 2;
-        int32_t q = e0 >> 2;
-        uint4 cur = q < q1 ? __ldg(codes4 + q) : null4;
-        for (; q < q1; ++q) {
-            const uint4 nxt = q + 1 < q1 ? __ldg(codes4 + q + 1) : null4;
-            const uint32_t code[4] = {cur.x, cur.y, cur.z, cur.w};
-            MxRaw<VM> val[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float* hi = nullptr;
-                const short* lo = nullptr;
-                val[u] = mx_entry(a, code[u], hi, lo) ? mx_ld<VM>(hi + c, lo + c) : mx_zero<VM>();
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (code[u] & GRG_B200_SEG_START) {
-                    add_into(acc, seg);
-                    seg = zero_pack<double, VM>();
-                }
-                mx_add<VM>(seg, val[u]);  // skipped entries decode to +0
-            }
-            cur = nxt;
-        }
-        add_into(acc, seg);
-        const int64_t off = row * a.ld_state + c;
-        mx_st<VM>(static_cast<float*>(a.state) + off, static_cast<short*>(a.state_lo) + off, acc);
-    }
-}
-
-// Heavy rows in mixed storage, one warp each (as level_warp_kernel, padded lists).
-template <int INIT, int VM>
-__global__ void __launch_bounds__(kWarpRowThreads) level_mx_warp_kernel(LevelArgs a) {
-    const int64_t w = static_cast<int64_t>(blockIdx.x) * (kWarpRowThreads / 32) + (threadIdx.x >> 5);
-    if (w >= a.num_heavy) return;  // warp-uniform
-    const int lane32 = threadIdx.x & 31;
-    const int64_t pos = __ldg(a.heavy_rows + w);
-    const int32_t e0 = __ldg(a.row_ptr + pos);
-    const int32_t e1 = __ldg(a.row_ptr + pos + 1);
-    const int64_t row = level_row(a, pos);
-    const int g_lanes = 1 << a.log2g;
-    const int groups = 32 >> a.log2g;
-    const int glane = lane32 & (g_lanes - 1);
-    const int grp = lane32 >> a.log2g;
-    const uint4* codes4 = reinterpret_cast<const uint4*>(a.entries);
-    const int64_t step = static_cast<int64_t>(VM) << a.log2g;
-    for (int64_t base = 0; base < a.k; base += step) {  // uniform trip count across the warp
-        const int64_t c = base + static_cast<int64_t>(glane) * VM;
-        const bool active = c < a.k;
-        Pack<double, VM> part = zero_pack<double, VM>();
-        if (active) {
-            for (int32_t q = (e0 >> 2) + grp; q < (e1 >> 2); q += groups) {
-                const uint4 cq = __ldg(codes4 + q);
-                const uint32_t code[4] = {cq.x, cq.y, cq.z, cq.w};
-                MxRaw<VM> val[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const float* hi = nullptr;
-                    const short* lo = nullptr;
-                    val[u] = mx_entry(a, code[u], hi, lo) ? mx_ld<VM>(hi + c, lo + c) : mx_zero<VM>();
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) mx_add<VM>(part, val[u]);
-            }
-        }
-        for (int off = 16; off >= g_lanes; off >>= 1) {
-            const Pack<double, VM> other = shfl_xor_pack(part, off);
-            add_into(part, other);
-        }
-        if (grp == 0 && active) {
-            Pack<double, VM> acc = mx_init_v<INIT, VM>(a, row, c);
-            add_into(acc, part);
-            const int64_t o = row * a.ld_state + c;
-            mx_st<VM>(static_cast<float*>(a.state) + o, static_cast<short*>(a.state_lo) + o, acc);
-        }
-    }
-}
-
 // Encoded copy of an FP64 matrix: dst[r, c] = src[r, c] for c < k, 0 for k <= c < ld.
 __global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, int64_t ld_src, int64_t rows, int64_t k,
-                                                             float* dst_hi, short* dst_lo, int64_t ld, int32_t log2g) {
+                                                             uint32_t* dst_hi, uint16_t* dst_lo, int64_t ld, int32_t log2g) {
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t r = t >> log2g;
     if (r >= rows) return;
@@ -1323,8 +999,8 @@ __global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, 
 }
 
 // Up seeding of level 0 in mixed storage: state[r] = init(r) (+ input row for samples).
-template <int INIT>
-__global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
+__global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, int init_mode, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
+    pdl_trigger();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t row = t >> a.log2g;
     if (row >= a.num_rows) return;
@@ -1339,10 +1015,10 @@ __global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, int64_t nu
     }
     const double* x = static_cast<const double*>(a.x);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
-        Quad v = mx_init<INIT>(a, row, c);
+        Quad v = mx_init(a, init_mode, row, c);
         if (row < num_samples) add_quad(v, f64_load_guarded(x + xrow * a.ld_x, c, a.k));
         const int64_t o = row * a.ld_state + c;
-        mx_store(static_cast<float*>(a.state) + o, static_cast<short*>(a.state_lo) + o, v);
+        mx_store(static_cast<uint32_t*>(a.state) + o, static_cast<uint16_t*>(a.state_lo) + o, v);
     }
 }
 
@@ -1796,11 +1472,12 @@ __device__ __forceinline__ void mx_apply_bias(const OutArgs& a, int64_t r, int64
 
 __device__ __forceinline__ Quad mx_state_row(const OutArgs& a, int64_t n, int64_t c) {
     const int64_t o = n * a.ld_state + c;
-    return mx_load(static_cast<const float*>(a.state) + o, static_cast<const short*>(a.state_lo) + o);
+    return mx_load(static_cast<const uint32_t*>(a.state) + o, static_cast<const uint16_t*>(a.state_lo) + o);
 }
 
 template <bool BIAS_PER_ENTRY>
 __global__ void __launch_bounds__(256) gather_out_mx_kernel(OutArgs a) {
+    pdl_wait();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t r = t >> a.log2g;
     if (r >= a.rows) return;
@@ -1825,6 +1502,7 @@ __global__ void __launch_bounds__(256) gather_out_mx_kernel(OutArgs a) {
 }
 
 __global__ void __launch_bounds__(256) copy_out_mx_kernel(OutArgs a) {
+    pdl_wait();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t r = t >> a.log2g;
     if (r >= a.rows) return;
@@ -1838,6 +1516,7 @@ __global__ void __launch_bounds__(256) copy_out_mx_kernel(OutArgs a) {
 }
 
 __global__ void __launch_bounds__(256) emit_all_mx_kernel(OutArgs a) {
+    pdl_wait();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t j = t >> a.log2g;
     if (j >= a.rows) return;
@@ -2249,44 +1928,6 @@ int launch_level_typed(const LevelArgs& la, int init_mode, bool exact, int varia
     return GRG_B200_OK;
 }
 
-template <int VM>
-int launch_level_mx_typed(const LevelArgs& la, int init_mode, cudaStream_t s) {
-    const int64_t narrow = la.num_rows - la.num_heavy;  // heavy positions form the suffix
-    if (narrow > 0) {
-        const int64_t warps = (narrow + (32 >> la.log2g) - 1) >> (5 - la.log2g);
-        const dim3 grid(static_cast<unsigned>((warps + kNarrowWarps - 1) / kNarrowWarps));
-        switch (init_mode) {
-            case 0: level_mx_kernel<0, VM><<<grid, kNarrowThreads, 0, s>>>(la); break;
-            case 1: level_mx_kernel<1, VM><<<grid, kNarrowThreads, 0, s>>>(la); break;
-            case 2: level_mx_kernel<2, VM><<<grid, kNarrowThreads, 0, s>>>(la); break;
-            default: level_mx_kernel<3, VM><<<grid, kNarrowThreads, 0, s>>>(la); break;
-        }
-        GRG_LAUNCH_CHECK("level_mx_kernel");
-    }
-    if (la.num_heavy > 0) {
-        constexpr int rows_per_cta = kWarpRowThreads / 32;
-        const dim3 grid(static_cast<unsigned>((la.num_heavy + rows_per_cta - 1) / rows_per_cta));
-        switch (init_mode) {
-            case 0: level_mx_warp_kernel<0, VM><<<grid, kWarpRowThreads, 0, s>>>(la); break;
-            case 1: level_mx_warp_kernel<1, VM><<<grid, kWarpRowThreads, 0, s>>>(la); break;
-            case 2: level_mx_warp_kernel<2, VM><<<grid, kWarpRowThreads, 0, s>>>(la); break;
-            default: level_mx_warp_kernel<3, VM><<<grid, kWarpRowThreads, 0, s>>>(la); break;
-        }
-        GRG_LAUNCH_CHECK("level_mx_warp_kernel");
-    }
-    return GRG_B200_OK;
-}
-
-// Mixed level launches: narrow_variant 7 walks rows with 2 columns per lane, others with 4.
-int launch_level_mx(LevelArgs la, int init_mode, int variant, cudaStream_t s) {
-    const int vm = variant == 7 || variant >= 11 ? 2 : 4;
-    const int64_t cols = (la.k + vm - 1) / vm;
-    int log2g = 0;
-    while ((1 << log2g) < cols && log2g < 5) ++log2g;
-    la.log2g = log2g;
-    return vm == 2 ? launch_level_mx_typed<2>(la, init_mode, s) : launch_level_mx_typed<4>(la, init_mode, s);
-}
-
 template <typename F>
 int dispatch(const grg_b200_traverse_args* a, const Shape& sh, F&& f) {
     if (a->dtype == GRG_B200_F64) {
@@ -2366,12 +2007,13 @@ int run_level(const grg_b200_traverse_args* a, const Shape& sh, const grg_b200_l
     const int rc = build_level_args(a, sh, L, blob, la);
     if (rc) return rc;
     const bool exact = a->exact_order != 0;
-    if (a->dtype == GRG_B200_MIXED) return launch_level_mx(la, a->init_mode, a->narrow_variant, s);
-    if ((a->launch_flags & GRG_B200_LAUNCH_WALK) && walk_serves(la, a->init_mode, exact)) {
+    const bool mixed = a->dtype == GRG_B200_MIXED;
+    if (mixed || ((a->launch_flags & GRG_B200_LAUNCH_WALK) && walk_serves(la, a->init_mode, exact))) {
         const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
         for (int i = 0; i < GRG_B200_LONG_CLASSES; ++i)
             if (L->long_rows[i] < 0 || L->long_rows[i] > L->num_heavy)
                 return grg_fail(GRG_B200_ERR_INVALID, "long_rows[%d] %lld outside [0, %lld]", i, (long long)L->long_rows[i], (long long)L->num_heavy);
+        if (mixed) return launch_walk_mixed(la, a->init_mode, L->num_entries, L->long_rows, pdl, s);
         return a->dtype == GRG_B200_F64 ? launch_walk<double>(la, L->num_entries, L->long_rows, pdl, s)
                                         : launch_walk<float>(la, L->num_entries, L->long_rows, pdl, s);
     }
@@ -2459,12 +2101,7 @@ int seed_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t 
     la.num_rows = a->level0_rows;
     const dim3 grid = grid_for(la.num_rows, la.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        switch (a->init_mode) {
-            case 0: seed_up_mx_kernel<0><<<grid, 256, 0, s>>>(la, a->num_samples, a->sample_to_individual, a->by_individual); break;
-            case 1: seed_up_mx_kernel<1><<<grid, 256, 0, s>>>(la, a->num_samples, a->sample_to_individual, a->by_individual); break;
-            case 2: seed_up_mx_kernel<2><<<grid, 256, 0, s>>>(la, a->num_samples, a->sample_to_individual, a->by_individual); break;
-            default: seed_up_mx_kernel<3><<<grid, 256, 0, s>>>(la, a->num_samples, a->sample_to_individual, a->by_individual); break;
-        }
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_mx_kernel, la, a->init_mode, a->num_samples, a->sample_to_individual, a->by_individual));
         GRG_LAUNCH_CHECK("seed_up_mx_kernel");
         return (int)GRG_B200_OK;
     }
@@ -2512,7 +2149,7 @@ int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_
     o.idx = a->sel_mut_idx;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        gather_out_mx_kernel<false><<<grid, 256, 0, s>>>(o);
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, o));
         GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_mut)");
         if (a->use_miss) {
             OutArgs m = o;
@@ -2521,7 +2158,7 @@ int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_
             m.out = a->miss;
             m.ld_out = a->ld_miss;
             m.bias_mode = GRG_B200_BIAS_NONE;
-            gather_out_mx_kernel<false><<<grid, 256, 0, s>>>(m);
+            GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, m));
             GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_miss)");
         }
         return (int)GRG_B200_OK;
@@ -2561,8 +2198,8 @@ int output_down_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStrea
     if (o.rows == 0) return GRG_B200_OK;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        if (a->by_individual) gather_out_mx_kernel<true><<<grid, 256, 0, s>>>(o);
-        else copy_out_mx_kernel<<<grid, 256, 0, s>>>(o);
+        if (a->by_individual) GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<true>, o));
+        else GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, copy_out_mx_kernel, o));
         GRG_LAUNCH_CHECK("output_down_mx");
         return (int)GRG_B200_OK;
     }
@@ -2584,7 +2221,7 @@ int emit_all_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t
     o.idx = a->inv_node_perm;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        emit_all_mx_kernel<<<grid, 256, 0, s>>>(o);
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, emit_all_mx_kernel, o));
         GRG_LAUNCH_CHECK("emit_all_mx_kernel");
         return (int)GRG_B200_OK;
     }
@@ -2689,13 +2326,13 @@ int encode_down_inputs(const grg_b200_traverse_args* a, const Shape& sh, cudaStr
     while ((1 << log2g) < (ld + 3) / 4 && log2g < 5) ++log2g;
     const dim3 grid = grid_for(a->num_mutations, log2g, 256);
     mx_encode_rows_kernel<<<grid, 256, 0, s>>>(static_cast<const double*>(a->input), a->ld_input, a->num_mutations, a->k,
-                                               static_cast<float*>(const_cast<void*>(la.x)),
-                                               static_cast<short*>(const_cast<void*>(la.x_lo)), ld, log2g);
+                                               static_cast<uint32_t*>(const_cast<void*>(la.x)),
+                                               static_cast<uint16_t*>(const_cast<void*>(la.x_lo)), ld, log2g);
     GRG_LAUNCH_CHECK("mx_encode_rows_kernel(input)");
     if (a->use_miss) {
         mx_encode_rows_kernel<<<grid, 256, 0, s>>>(static_cast<const double*>(a->miss), a->ld_miss, a->num_mutations, a->k,
-                                                   static_cast<float*>(const_cast<void*>(la.miss)),
-                                                   static_cast<short*>(const_cast<void*>(la.miss_lo)), ld, log2g);
+                                                   static_cast<uint32_t*>(const_cast<void*>(la.miss)),
+                                                   static_cast<uint16_t*>(const_cast<void*>(la.miss_lo)), ld, log2g);
         GRG_LAUNCH_CHECK("mx_encode_rows_kernel(miss)");
     }
     return GRG_B200_OK;

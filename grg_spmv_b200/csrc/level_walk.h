@@ -1,4 +1,4 @@
-// The row walk of default-mode level launches (level_walk.cu).
+// The row walk of default-mode level launches (level_walk.cu) and of mixed storage (level_walk_mixed.cu).
 #ifndef GRG_B200_LEVEL_WALK_H
 #define GRG_B200_LEVEL_WALK_H
 
@@ -13,5 +13,9 @@ bool walk_serves(const LevelArgs& la, int init_mode, bool exact);
 // listed first in heavy_rows; nullptr when the level does not say.
 template <typename T>
 int launch_walk(const LevelArgs& la, int64_t num_entries, const int64_t* long_counts, bool pdl, cudaStream_t s);
+
+// The same over mixed storage, for every launch of that dtype (any init, with or without an error
+// word).
+int launch_walk_mixed(const LevelArgs& la, int init_mode, int64_t num_entries, const int64_t* long_counts, bool pdl, cudaStream_t s);
 
 #endif  // GRG_B200_LEVEL_WALK_H

@@ -66,11 +66,12 @@ typedef enum grg_b200_status {
 
 /*
  * GRG_B200_MIXED: input, output, miss and init buffers are FP64; the node state (and, for
- * down, encoded copies of input and miss in mix_scratch) is stored in 6 bytes per value:
- * hi = the value rounded to FP32 and lo = a 16-bit correction in units of 2^(e(hi) - 38), so
- * a stored value is within 2^-39 of the exact one relative to |hi| (integers below 2^39 are
+ * down, encoded copies of input and miss in mix_scratch) is stored in 6 bytes per value: hi, the
+ * leading 32 bits of the value as an FP32 number (sign, exponent, 23 mantissa bits, truncated),
+ * and lo, the next 16 mantissa bits.  The value is rounded to these 40 significant bits, so a
+ * stored value is within 2^-40 of the exact one relative to it (integers up to 2^40 are
  * exact).  Sums are accumulated in FP64 and rounded back once per node.  A mixed buffer of
- * R rows and ld columns (ld a multiple of 4) is float hi[R * ld] followed by int16
+ * R rows and ld columns (ld a multiple of 4) is uint32 hi[R * ld] followed by uint16
  * lo[R * ld]; see GRG_B200_MIX_BYTES.  Mixed traversals never use exact order.
  */
 typedef enum grg_b200_dtype { GRG_B200_F64 = 0, GRG_B200_F32 = 1, GRG_B200_MIXED = 2 } grg_b200_dtype;
