@@ -189,6 +189,9 @@ EXPORTED_SYMBOLS = (
     "grg_b200_traverse",
     "grg_b200_traverse_static",
     "grg_b200_rowop",
+    "grg_b200_graph_create",
+    "grg_b200_graph_launch",
+    "grg_b200_graph_destroy",
 )
 
 _lock = threading.Lock()
@@ -250,6 +253,11 @@ def load_library():
         for name in ("grg_b200_seed_up", "grg_b200_output_up", "grg_b200_output_down", "grg_b200_emit_all", "grg_b200_traverse",
                      "grg_b200_traverse_static"):
             getattr(lib, name).argtypes = [ctypes.POINTER(TraverseArgs), ctypes.c_void_p]
+            getattr(lib, name).restype = ctypes.c_int
+        lib.grg_b200_graph_create.argtypes = [ctypes.POINTER(TraverseArgs), ctypes.POINTER(ctypes.c_void_p)]
+        lib.grg_b200_graph_launch.argtypes = [ctypes.c_void_p, ctypes.POINTER(TraverseArgs), ctypes.c_void_p]
+        lib.grg_b200_graph_destroy.argtypes = [ctypes.c_void_p]
+        for name in ("grg_b200_graph_create", "grg_b200_graph_launch", "grg_b200_graph_destroy"):
             getattr(lib, name).restype = ctypes.c_int
         lib.grg_b200_rowop.argtypes = [ctypes.POINTER(RowopArgs), ctypes.c_void_p]
         lib.grg_b200_rowop.restype = ctypes.c_int

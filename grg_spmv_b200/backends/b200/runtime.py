@@ -76,8 +76,27 @@ class _DeviceArtifact:
     level0_rows: int
 
 
+class _Recording:
+    """A traversal recorded as a CUDA graph (``grg_b200_graph_*``), destroyed with its owner."""
+
+    def __init__(self, lib, args: nat.TraverseArgs) -> None:
+        self._lib = lib
+        self._handle = ctypes.c_void_p()
+        nat.check(lib, lib.grg_b200_graph_create(ctypes.byref(args), ctypes.byref(self._handle)), "grg_b200_graph_create")
+
+    def launch(self, args: nat.TraverseArgs, stream_ptr: int) -> int:
+        return self._lib.grg_b200_graph_launch(self._handle, args, stream_ptr)
+
+    def __del__(self) -> None:
+        if getattr(self, "_handle", None):
+            self._lib.grg_b200_graph_destroy(self._handle)
+
+
 class B200PreparedMatmul:
-    def __init__(self, runtime: "B200Runtime", artifact: _DeviceArtifact, spec: CudaMatmulSpec) -> None:
+    """``record=False`` prepares a single call: it launches its kernels one by one (recording them
+    first costs several times as much as one such call)."""
+
+    def __init__(self, runtime: "B200Runtime", artifact: _DeviceArtifact, spec: CudaMatmulSpec, record: bool = True) -> None:
         self._runtime = runtime
         self._artifact = artifact
         self._spec = spec
@@ -110,7 +129,7 @@ class B200PreparedMatmul:
             self.init_matrix = init_matrix.T
         self._args = runtime._traverse_args(artifact, spec, self._input_internal, self._output_internal, miss_view,
                                             init_vector, init_matrix)
-        self._graph = runtime._capture(self._args)
+        self._graph = runtime._capture(self._args) if record else None
 
     def __enter__(self) -> "B200PreparedMatmul":
         return self
@@ -119,8 +138,12 @@ class B200PreparedMatmul:
         return None
 
     def __call__(self) -> None:
-        with self._runtime._call_scope():
-            self._call_prelocked()
+        runtime = self._runtime
+        runtime._begin_call()
+        try:
+            runtime._launch(self._args, self._graph)
+        finally:
+            runtime._active_call = False
 
     def _call_prelocked(self) -> None:
         self._runtime._launch(self._args, self._graph)
@@ -410,26 +433,33 @@ class B200Runtime:
     def _torch_caller_stream(self):
         return self._caller_stream
 
-    @contextmanager
-    def _call_scope(self):
+    def _begin_call(self) -> None:
         if not self._entered:
             raise RuntimeError("B200Runtime must be entered before matmul")
         if self._active_call:
             raise RuntimeError("concurrent runtime.grgs calls are not supported")
         self._active_call = True
+
+    @contextmanager
+    def _call_scope(self):
+        self._begin_call()
         try:
             yield
         finally:
             self._active_call = False
 
-    def _prepare_matmul_cuda(self, grg, spec) -> B200PreparedMatmul:
+    def _prepare_once(self, grg, spec) -> B200PreparedMatmul:
+        """A prepared op for one call (``BoundGRG.matmul``)."""
+        return self._prepare_matmul_cuda(grg, spec, record=False)
+
+    def _prepare_matmul_cuda(self, grg, spec, record: bool = True) -> B200PreparedMatmul:
         if spec.direction == Direction.UP and self.layout.pair.plan_up is None:
             raise ValueError("UP plan is not configured")
         if spec.direction == Direction.DOWN and self.layout.pair.plan_down is None:
             raise ValueError("DOWN plan is not configured")
         if spec.emit_all_nodes and not self.layout.emit_all_nodes:
             raise ValueError("emit_all_nodes needs a layout planned with emit_all_nodes=True")
-        return B200PreparedMatmul(self, self._artifacts[int(grg._artifact_index)], spec)
+        return B200PreparedMatmul(self, self._artifacts[int(grg._artifact_index)], spec, record)
 
     def _traverse_args(self, art: _DeviceArtifact, spec, input_view, output_view, miss_view, init_vector, init_matrix, *,
                        state=None, mixed: bool | None = None, mix_scratch=None, df_sync=None):
@@ -532,27 +562,18 @@ class B200Runtime:
         if not self._use_graphs or self._capturing():
             return None
         with torch.cuda.device(self.device):
-            graph = torch.cuda.CUDAGraph()
-            side = torch.cuda.Stream(device=self.device)
-            with torch.cuda.stream(side):
-                graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    status = self._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(side.cuda_stream))
-                finally:
-                    graph.capture_end()
-        nat.check(self._lib, status, "grg_b200_traverse (graph capture)")
-        return graph
+            return _Recording(self._lib, args)
 
-    def _launch(self, args: nat.TraverseArgs, graph=None) -> None:
-        import torch
+    def _launch(self, args: nat.TraverseArgs, recording: _Recording | None = None) -> None:
+        if recording is not None:
+            status = recording.launch(args, self.stream_ptr)
+        else:
+            import torch
 
-        with torch.cuda.device(self.device):
-            if graph is not None and not self._capturing():
-                with torch.cuda.stream(self._caller_stream):
-                    graph.replay()
-                return
-            status = self._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(self.stream_ptr))
-        nat.check(self._lib, status, "grg_b200_traverse")
+            with torch.cuda.device(self.device):
+                status = self._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(self.stream_ptr))
+        if status != nat.OK:
+            nat.check(self._lib, status, "grg_b200_traverse")
 
     def prepare_batch(self, items, *, precision: str | None = None, tile_k: int | None = None, autotune: bool = False):
         """Several (grg, direction, k) matmuls run together as one CUDA graph; see

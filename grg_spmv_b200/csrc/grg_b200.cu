@@ -31,6 +31,7 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <type_traits>
 
 #include "level_common.cuh"
@@ -2628,6 +2629,84 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
     if (a->emit_all_nodes) return emit_all_impl(a, sh, s);
     if (a->direction == GRG_B200_UP) return output_up_impl(a, sh, s);
     return output_down_impl(a, sh, s);
+}
+
+// ---------------------------------------------------------------------------------------
+// Recorded traversals: a level launch costs the host 2 to 3 us and the GPU a gap of its own, a
+// recorded traversal one launch (about 5 us for 20 to 40 levels).
+// ---------------------------------------------------------------------------------------
+}  // extern "C"
+
+struct grg_b200_graph {
+    int device;
+    cudaGraphExec_t exec;
+};
+
+namespace {
+// Makes `device` current for a scope.
+struct DeviceScope {
+    int previous = -1;
+    cudaError_t status;
+    explicit DeviceScope(int device) {
+        status = cudaGetDevice(&previous);
+        if (status == cudaSuccess && previous != device) status = cudaSetDevice(device);
+        else previous = -1;
+    }
+    ~DeviceScope() {
+        if (previous >= 0) cudaSetDevice(previous);
+    }
+};
+}  // namespace
+
+extern "C" {
+
+int grg_b200_graph_create(const grg_b200_traverse_args* a, grg_b200_graph** out) {
+    if (!out) return grg_fail(GRG_B200_ERR_INVALID, "graph out pointer is NULL");
+    *out = nullptr;
+    int device = 0;
+    GRG_CUDA_TRY(cudaGetDevice(&device));
+    cudaStream_t side = nullptr;
+    GRG_CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    int rc = GRG_B200_OK;
+    cudaError_t err = cudaStreamBeginCapture(side, cudaStreamCaptureModeThreadLocal);
+    if (err == cudaSuccess) {
+        rc = grg_b200_traverse(a, side);
+        err = cudaStreamEndCapture(side, &graph);
+        if (rc == GRG_B200_OK && err == cudaSuccess) err = cudaGraphInstantiate(&exec, graph, 0);
+    }
+    if (graph) cudaGraphDestroy(graph);
+    cudaStreamDestroy(side);
+    if (rc != GRG_B200_OK) return rc;
+    if (err != cudaSuccess) return grg_fail(GRG_B200_ERR_CUDA, "recording a traversal failed: %s", cudaGetErrorString(err));
+    grg_b200_graph* g = new (std::nothrow) grg_b200_graph{device, exec};
+    if (!g) {
+        cudaGraphExecDestroy(exec);
+        return grg_fail(GRG_B200_ERR_CUDA, "out of host memory");
+    }
+    *out = g;
+    return GRG_B200_OK;
+}
+
+int grg_b200_graph_launch(const grg_b200_graph* g, const grg_b200_traverse_args* a, void* stream_handle) {
+    if (!g) return grg_fail(GRG_B200_ERR_INVALID, "graph is NULL");
+    cudaStream_t s = static_cast<cudaStream_t>(stream_handle);
+    const DeviceScope scope(g->device);
+    GRG_CUDA_TRY(scope.status);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    GRG_CUDA_TRY(cudaStreamIsCapturing(s, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return grg_b200_traverse(a, stream_handle);
+    GRG_CUDA_TRY(cudaGraphLaunch(g->exec, s));
+    return GRG_B200_OK;
+}
+
+int grg_b200_graph_destroy(grg_b200_graph* g) {
+    if (!g) return GRG_B200_OK;
+    const DeviceScope scope(g->device);
+    const cudaError_t err = cudaGraphExecDestroy(g->exec);
+    delete g;
+    return err == cudaSuccess ? (int)GRG_B200_OK : grg_fail(GRG_B200_ERR_CUDA, "cudaGraphExecDestroy failed: %s", cudaGetErrorString(err));
 }
 
 // ---------------------------------------------------------------------------------------

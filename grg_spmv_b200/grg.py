@@ -249,8 +249,8 @@ class BoundGRG:
         if stream is None:
             return src.detach().cpu().numpy().astype(self._dtype, copy=False).copy()
         with torch.cuda.device(src.device), torch.cuda.stream(stream()):
-            host = src.detach().cpu()
-        return host.numpy().astype(self._dtype, copy=False).copy()
+            host = src.detach().contiguous().cpu()  # rows put in order on the GPU, not by a host copy
+        return host.numpy().astype(self._dtype, copy=False)
 
     def matmul(self, input, direction, emit_all_nodes: bool = False, by_individual: bool = False, init=None, miss=None):
         if not isinstance(input, np.ndarray):
@@ -279,9 +279,10 @@ class BoundGRG:
         spec = self._prepare_cuda_spec(direction=direction, k=rows, emit_all_nodes=bool(emit_all_nodes),
                                        by_individual=bool(by_individual), init_mode=init_mode, use_miss=miss is not None)
         miss_matrix = None if miss is None else self._validate_miss(miss, rows, direction, input.dtype)
+        # a runtime that records prepared ops (B200Runtime) prepares this one call without
+        prepare = getattr(self._runtime, "_prepare_once", self._runtime._prepare_matmul_cuda)
         with self._runtime._call_scope():
-            with self.prepare_matmul_cuda(direction=spec.direction, k=spec.k, emit_all_nodes=spec.emit_all_nodes,
-                                          by_individual=spec.by_individual, init_mode=spec.init_mode, use_miss=spec.use_miss) as op:
+            with prepare(self, spec) as op:
                 self._copy_host_to_cuda(op.input, input)
                 if spec.direction == Direction.DOWN and miss_matrix is not None:
                     self._copy_host_to_cuda(op.miss_input, miss_matrix)

@@ -378,6 +378,18 @@ typedef struct grg_b200_rowop_args {
     ((((rows) + 255) / 256) < GRG_B200_ROWOP_MAX_BLOCKS ? (((rows) + 255) / 256) : GRG_B200_ROWOP_MAX_BLOCKS)
 int grg_b200_rowop(const grg_b200_rowop_args* args, void* stream);
 
+/* A traversal recorded as a CUDA graph (no counterpart in the reference, whose prepared calls
+ * launch block by block).  create records grg_b200_traverse(args) on a stream of its own on the
+ * current device; the recording holds args' pointers, sizes and level blobs, which must stay
+ * valid.  launch replays it on `stream` with one launch; while that stream is being captured it
+ * issues the traversal's kernels into the capture instead.  A recording may be launched from any
+ * thread, one call at a time; destroy waits for nothing and takes effect once its launches are
+ * done. */
+typedef struct grg_b200_graph grg_b200_graph;
+int grg_b200_graph_create(const grg_b200_traverse_args* args, grg_b200_graph** out);
+int grg_b200_graph_launch(const grg_b200_graph* graph, const grg_b200_traverse_args* args, void* stream);
+int grg_b200_graph_destroy(grg_b200_graph* graph);
+
 /* No counterpart in the reference.  The same traversal as grg_b200_traverse for callers that
  * cannot allocate device memory (C/FFI hosts without a device allocator, plugins inside
  * another framework's memory manager, code that must not allocate during stream capture):
