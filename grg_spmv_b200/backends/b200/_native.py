@@ -173,7 +173,7 @@ ROWOP_MAX_BLOCKS = 1184
 
 def rowop_blocks(rows: int) -> int:
     """GRG_B200_ROWOP_BLOCKS: row blocks (and rows of partial sums) of a rowop call."""
-    return min((int(rows) + 255) // 256, ROWOP_MAX_BLOCKS)
+    return min((int(rows) + 31) // 32, ROWOP_MAX_BLOCKS)
 
 
 EXPORTED_SYMBOLS = (

@@ -39,9 +39,9 @@ def _ptr(t) -> int | None:
 
 
 class _RowStep:
-    """One ``grg_b200_rowop`` pass with fixed buffers (the source may change per call)."""
+    """One ``grg_b200_rowop`` pass with fixed buffers (source and destination may change per call)."""
 
-    def __init__(self, lib, stream_ptr: int, *, rows: int, k: int, src=None, dst, miss_in=None, miss_scale=None,
+    def __init__(self, lib, stream_ptr: int, *, rows: int, k: int, src=None, dst=None, miss_in=None, miss_scale=None,
                  pre_scale=None, col_sub=None, sub_scale=None, post_scale=None, miss_out=None, miss_out_scale=None,
                  sums=None, sum_weight=None, partials=None) -> None:
         self._lib = lib
@@ -52,9 +52,11 @@ class _RowStep:
                                   miss_out_scale=_ptr(miss_out_scale), col_sums=int(sums is not None),
                                   sum_weight=_ptr(sum_weight), partials=_ptr(partials), sums=_ptr(sums))
 
-    def __call__(self, src=None) -> None:
+    def __call__(self, src=None, dst=None) -> None:
         if src is not None:
             self.args.src = int(src.data_ptr())
+        if dst is not None:
+            self.args.dst = int(dst.data_ptr())
         nat.check(self._lib, self._lib.grg_b200_rowop(ctypes.byref(self.args), self._stream), "grg_b200_rowop")
 
 
@@ -69,7 +71,7 @@ class StandardizedXTX:
         self.q = int(q)
         self.has_missing = bool(grg.has_missing_data)
         self.shape = (int(grg.num_mutations), int(grg.num_mutations))
-        dev = torch.device(runtime.device)
+        dev = self._device = torch.device(runtime.device)
         self._stream = runtime._torch_caller_stream()
         with torch.cuda.device(dev), torch.cuda.stream(self._stream):
             ones_op = grg.prepare_matmul_cuda(direction="up", k=1, by_individual=True, use_miss=self.has_missing)
@@ -90,7 +92,6 @@ class StandardizedXTX:
             self.center_over_sigma = self.center * self.inv_sigma
             self._down = grg.prepare_matmul_cuda(direction="down", k=self.q, by_individual=True, use_miss=self.has_missing)
             self._up = grg.prepare_matmul_cuda(direction="up", k=self.q, by_individual=True, use_miss=self.has_missing)
-            self._out = torch.empty((self.shape[0], self.q), device=dev, dtype=torch.float64)
             M, I = int(grg.num_mutations), int(grg.num_individuals)
             self._partials = torch.empty((nat.rowop_blocks(max(M, I)), self.q), device=dev, dtype=torch.float64)
             self.c_down = torch.empty(self.q, device=dev, dtype=torch.float64)
@@ -105,7 +106,7 @@ class StandardizedXTX:
         self._center = _RowStep(lib, sp, rows=I, k=self.q, src=down.output, dst=up.input, col_sub=self.c_down,
                                 sums=self.c_up, partials=self._partials)
         # out = (up(u) + p * up_miss) / sigma - c_up * centre / sigma
-        self._finish = _RowStep(lib, sp, rows=M, k=self.q, src=up.output, dst=self._out,
+        self._finish = _RowStep(lib, sp, rows=M, k=self.q, src=up.output,
                                 miss_in=up.miss_output if miss else None, miss_scale=self.freqs if miss else None,
                                 pre_scale=self.inv_sigma, col_sub=self.c_up, sub_scale=self.center_over_sigma)
 
@@ -115,7 +116,7 @@ class StandardizedXTX:
 
         if tuple(v.shape) != (self.shape[0], self.q):
             raise ValueError(f"operand has shape {tuple(v.shape)}, expected ({self.shape[0]}, {self.q})")
-        if v.dtype != torch.float64 or v.device != self._out.device:
+        if v.dtype != torch.float64 or v.device != self._device:
             raise ValueError("operand must be a float64 tensor on the runtime's device")
         with torch.cuda.stream(self._stream):
             v = v.contiguous()
@@ -123,8 +124,9 @@ class StandardizedXTX:
             self._down()
             self._center()
             self._up()
-            self._finish()
-            return self._out.clone()
+            out = torch.empty_like(v)
+            self._finish(dst=out)
+            return out
 
 
 class StandardizedXXT:
@@ -138,7 +140,6 @@ class StandardizedXXT:
         self._xtx = StandardizedXTX(runtime, grg, q)
         self.q = int(q)
         self.shape = (int(grg.num_individuals), int(grg.num_individuals))
-        self._out = torch.empty(self.shape[0], self.q, device=self._xtx._out.device, dtype=torch.float64)
         x = self._xtx
         lib, sp = runtime._lib, int(x._stream.cuda_stream)
         down, up, miss = x._down, x._up, x.has_missing
@@ -153,7 +154,7 @@ class StandardizedXXT:
                              miss_out=down.miss_input if miss else None, miss_out_scale=x.freqs if miss else None,
                              sums=x.c_down, sum_weight=x.center, partials=x._partials)
         # out = down(d) - c_down
-        self._finish = _RowStep(lib, sp, rows=I, k=self.q, src=down.output, dst=self._out, col_sub=x.c_down)
+        self._finish = _RowStep(lib, sp, rows=I, k=self.q, src=down.output, col_sub=x.c_down)
 
     def apply(self, w):
         import torch
@@ -161,7 +162,7 @@ class StandardizedXXT:
         x = self._xtx
         if tuple(w.shape) != (self.shape[0], self.q):
             raise ValueError(f"operand has shape {tuple(w.shape)}, expected ({self.shape[0]}, {self.q})")
-        if w.dtype != torch.float64 or w.device != self._out.device:
+        if w.dtype != torch.float64 or w.device != x._device:
             raise ValueError("operand must be a float64 tensor on the runtime's device")
         with torch.cuda.stream(x._stream):
             w = w.contiguous()
@@ -169,8 +170,9 @@ class StandardizedXXT:
             x._up()
             self._mid()
             x._down()
-            self._finish()
-            return self._out.clone()
+            out = torch.empty_like(w)
+            self._finish(dst=out)
+            return out
 
 
 def conj_grad_solve(matvec, rhs, *, rel_tol: float, max_iter: int, project=None):

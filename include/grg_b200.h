@@ -371,11 +371,11 @@ typedef struct grg_b200_rowop_args {
     double* sums;
 } grg_b200_rowop_args;
 
-/* Row blocks of a rowop call: one per 256 rows, at most 1184 (the partial sums hold one row of
+/* Row blocks of a rowop call: one per 32 rows, at most 1184 (the partial sums hold one row of
  * k doubles per block). */
 #define GRG_B200_ROWOP_MAX_BLOCKS 1184
 #define GRG_B200_ROWOP_BLOCKS(rows) \
-    ((((rows) + 255) / 256) < GRG_B200_ROWOP_MAX_BLOCKS ? (((rows) + 255) / 256) : GRG_B200_ROWOP_MAX_BLOCKS)
+    ((((rows) + 31) / 32) < GRG_B200_ROWOP_MAX_BLOCKS ? (((rows) + 31) / 32) : GRG_B200_ROWOP_MAX_BLOCKS)
 int grg_b200_rowop(const grg_b200_rowop_args* args, void* stream);
 
 /* A traversal recorded as a CUDA graph (no counterpart in the reference, whose prepared calls
