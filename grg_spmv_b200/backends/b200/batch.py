@@ -32,6 +32,7 @@ from grg_spmv_b200.grg import CudaMatmulSpec
 from grg_spmv_b200.types import Direction, InitMode
 
 from . import _native as nat
+from .plan import state_ld
 
 
 @dataclass(frozen=True)
@@ -169,7 +170,7 @@ class B200BatchedMatmul:
                         nbytes = nat.mix_bytes(st.num_mutations, nat.mix_ld(w)) * (2 if g.use_miss else 1)
                         scratch = torch.zeros(nbytes, device=rt.device, dtype=torch.uint8)
                 else:
-                    state = torch.zeros(st.num_nodes * w, device=rt.device, dtype=self._tdt)
+                    state = torch.zeros(st.num_nodes * state_ld(w, rt.layout.dtype.itemsize), device=rt.device, dtype=self._tdt)
                     scratch = None
                 spec = CudaMatmulSpec(direction=g.direction, k=w, emit_all_nodes=False, by_individual=False,
                                       init_mode=InitMode.NONE, backend_init_mode=InitMode.NONE, use_miss=g.use_miss,

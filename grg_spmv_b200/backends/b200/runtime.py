@@ -32,7 +32,7 @@ import numpy as np
 
 from grg_spmv_b200.artifact import iter_artifact_blocks, load_grg_spmv_header
 from grg_spmv_b200.backends.b200 import _native as nat
-from grg_spmv_b200.backends.b200.plan import B200Layout, side_io_rows
+from grg_spmv_b200.backends.b200.plan import B200Layout, side_io_rows, state_ld
 from grg_spmv_b200.backends.b200.structures import build_down_levels, build_up_levels, load_blocks
 from grg_spmv_b200.grg import BoundGRG, CudaMatmulSpec
 from grg_spmv_b200.types import Direction, InitMode
@@ -234,7 +234,7 @@ class B200Runtime:
                     if lay.mix_scratch_bytes:
                         self._mix_scratch = torch.zeros(lay.mix_scratch_bytes, device=self.device, dtype=torch.uint8)
                 else:
-                    self._state = torch.zeros(lay.max_num_nodes * max_k, device=self.device, dtype=tdt)
+                    self._state = torch.zeros(lay.max_num_nodes * lay.state_ld, device=self.device, dtype=tdt)
                 self._io0 = torch.zeros((max(lay.max_num_samples, lay.max_num_mutations), max_k), device=self.device, dtype=tdt)
                 io1_rows = side_io_rows(lay.pair, lay.requirements, max_num_mutations=lay.max_num_mutations,
                                         max_num_nodes=lay.max_num_nodes)
@@ -497,7 +497,11 @@ class B200Runtime:
         a.num_mutations = st.num_mutations
         a.num_individuals = st.num_individuals
         a.state = _ptr(state)
-        a.ld_state = nat.mix_ld(k) if mixed else k
+        if mixed:
+            a.ld_state = nat.mix_ld(k)
+        else:  # whole vectors a row, where the state was planned with room for them
+            padded = state_ld(k, self.layout.dtype.itemsize)
+            a.ld_state = padded if state.numel() >= st.num_nodes * padded else k
         if mixed and mix_scratch is not None:
             a.mix_scratch = _ptr(mix_scratch)
             a.mix_scratch_bytes = int(mix_scratch.numel())

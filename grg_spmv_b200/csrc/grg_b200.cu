@@ -1332,9 +1332,47 @@ __global__ void __launch_bounds__(256) sentinel_fill_kernel(T* state, int64_t n)
         out[i] = bits;
 }
 
+// Columns [c, c + V) of an input or output row: one vector where `vec` says that k, the strides and
+// the bases allow it, else value by value up to k.  State rows hold whole vectors either way.
+template <typename T, int V>
+__device__ __forceinline__ Pack<T, V> ld_io(const T* row, int64_t c, int64_t k, bool vec) {
+    if (vec) return ld_ro<T, V>(row + c);
+    Pack<T, V> r;
+#pragma unroll
+    for (int i = 0; i < V; ++i) r.v[i] = c + i < k ? __ldg(row + c + i) : T(0);
+    return r;
+}
+
+template <typename T, int V>
+__device__ __forceinline__ void st_io(T* row, int64_t c, int64_t k, bool vec, const Pack<T, V>& x) {
+    if (vec) {
+        st_pack(row + c, x);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+        if (c + i < k) row[c + i] = x.v[i];
+}
+
+template <typename T, int V, int INIT>
+__device__ __forceinline__ Pack<T, V> init_io(const LevelArgs& a, int64_t row, int64_t c, bool vec) {
+    if constexpr (INIT == GRG_B200_INIT_VECTOR) {
+        return ld_io<T, V>(static_cast<const T*>(a.init_vector), c, a.k, vec);
+    } else if constexpr (INIT == GRG_B200_INIT_MATRIX) {
+        const int64_t orig = __ldg(a.node_perm + row);
+        if (a.err && (orig < 0 || orig >= a.lim_state)) {
+            report(a.err, kErrPerm);
+            return zero_pack<T, V>();
+        }
+        return ld_io<T, V>(static_cast<const T*>(a.init_matrix) + orig * a.ld_init, c, a.k, vec);
+    } else {
+        return init_value<T, V, INIT>(a, row, c);
+    }
+}
+
 // Up seeding of level 0: state[r] = init(r) (+ input row for samples).
 template <typename T, int V, int INIT>
-__global__ void __launch_bounds__(256) seed_up_kernel(LevelArgs a, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
+__global__ void __launch_bounds__(256) seed_up_kernel(LevelArgs a, bool vec, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
     pdl_trigger();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t row = t >> a.log2g;
@@ -1352,8 +1390,8 @@ __global__ void __launch_bounds__(256) seed_up_kernel(LevelArgs a, int64_t num_s
     pdl_wait();  // inputs, init values and the state it overwrites belong to earlier kernels
     const int64_t step = static_cast<int64_t>(V) << a.log2g;
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step) {
-        Pack<T, V> v = init_value<T, V, INIT>(a, row, c);
-        if (row < num_samples) add_into(v, ld_ro<T, V>(static_cast<const T*>(a.x) + xrow * a.ld_x + c));
+        Pack<T, V> v = init_io<T, V, INIT>(a, row, c, vec);
+        if (row < num_samples) add_into(v, ld_io<T, V>(static_cast<const T*>(a.x) + xrow * a.ld_x, c, a.k, vec));
         st_pack(state + row * a.ld_state + c, v);
     }
 }
@@ -1371,6 +1409,7 @@ struct OutArgs {
     int32_t bias_mode;
     int64_t k;
     int32_t log2g;
+    bool vec;              // output (and init vector) rows take whole vectors
     int32_t* err;
     int64_t lim;
     const void* state_lo;  // mixed storage only
@@ -1384,38 +1423,72 @@ __device__ __forceinline__ void apply_bias(const OutArgs& a, int64_t r, int64_t 
         for (int i = 0; i < V; ++i) v.v[i] = add_rn(v.v[i], b);
     } else if (a.bias_mode == GRG_B200_BIAS_VECTOR) {
         const T b = __ldg(static_cast<const T*>(a.bias) + r);
-        const Pack<T, V> iv = ld_ro<T, V>(static_cast<const T*>(a.init_vector) + c);
+        const Pack<T, V> iv = ld_io<T, V>(static_cast<const T*>(a.init_vector), c, a.k, a.vec);
 #pragma unroll
         for (int i = 0; i < V; ++i) v.v[i] = add_rn(v.v[i], mul_rn(b, iv.v[i]));
     }
 }
 
-// out[r] = sum over idx[ptr[r]..ptr[r+1]) of state rows (from zero, in order) + bias.
-template <typename T, int V, bool BIAS_PER_ENTRY>
+// out[r] = sum over idx[ptr[r]..ptr[r+1]) of state rows (from zero, in order) + bias.  Bound by
+// memory: most rows name one state row, so a lane group takes R rows, loads their extents and
+// first indexes before the wait (the lists are static) and keeps their first state rows in flight
+// together.  R = 1 while the rows fit the GPU at once: 4 would leave it idle (2,000 x 1: +2 us),
+// beyond that 1M x 8 takes 31 us instead of 37.
+constexpr int kOutRows = 4;
+
+template <typename T, int V, bool BIAS_PER_ENTRY, int R>
 __global__ void __launch_bounds__(256) gather_out_kernel(OutArgs a) {
+    const int per_block = 256 >> a.log2g;
+    const int lane = static_cast<int>(threadIdx.x) & ((1 << a.log2g) - 1);
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * per_block * R + (threadIdx.x >> a.log2g);
+    int32_t e0[R], e1[R];
+    int64_t n0[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const int64_t r = first + static_cast<int64_t>(u) * per_block;
+        e0[u] = r < a.rows ? __ldg(a.ptr + r) : 0;
+        e1[u] = r < a.rows ? __ldg(a.ptr + r + 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) n0[u] = e0[u] < e1[u] ? __ldg(a.idx + e0[u]) : 0;
     pdl_wait();
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t r = t >> a.log2g;
-    if (r >= a.rows) return;
-    const int lane = static_cast<int>(t & ((1 << a.log2g) - 1));
-    const int32_t e0 = __ldg(a.ptr + r), e1 = __ldg(a.ptr + r + 1);
     const T* state = static_cast<const T*>(a.state);
     T* out = static_cast<T*>(a.out);
     const int64_t step = static_cast<int64_t>(V) << a.log2g;
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step) {
-        Pack<T, V> s = zero_pack<T, V>();
-        for (int32_t e = e0; e < e1; ++e) {
-            const int64_t n = __ldg(a.idx + e);
-            if (a.err && (n < 0 || n >= a.lim)) {
-                report(a.err, kErrSelector);
-                continue;
+        Pack<T, V> v[R];
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            v[u] = zero_pack<T, V>();
+            if (e0[u] < e1[u]) {
+                if (a.err && (n0[u] < 0 || n0[u] >= a.lim)) report(a.err, kErrSelector);
+                else v[u] = ld_ro<T, V>(state + n0[u] * a.ld_state + c);
             }
-            Pack<T, V> v = ld_ro<T, V>(state + n * a.ld_state + c);
-            if constexpr (BIAS_PER_ENTRY) apply_bias<T, V>(a, n, c, v);  // down by individual
-            add_into(s, v);
         }
-        if constexpr (!BIAS_PER_ENTRY) apply_bias<T, V>(a, r, c, s);
-        st_pack(out + r * a.ld_out + c, s);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int64_t r = first + static_cast<int64_t>(u) * per_block;
+            if (r < a.rows) {
+                Pack<T, V> s = zero_pack<T, V>();
+                for (int32_t e = e0[u]; e < e1[u]; ++e) {
+                    int64_t n = n0[u];
+                    if (e > e0[u]) {
+                        n = __ldg(a.idx + e);
+                        if (a.err && (n < 0 || n >= a.lim)) {
+                            report(a.err, kErrSelector);
+                            continue;
+                        }
+                        v[u] = ld_ro<T, V>(state + n * a.ld_state + c);
+                    } else if (a.err && (n < 0 || n >= a.lim)) {
+                        continue;
+                    }
+                    if constexpr (BIAS_PER_ENTRY) apply_bias<T, V>(a, n, c, v[u]);  // down by individual
+                    add_into(s, v[u]);
+                }
+                if constexpr (!BIAS_PER_ENTRY) apply_bias<T, V>(a, r, c, s);
+                st_io(out + r * a.ld_out, c, a.k, a.vec, s);
+            }
+        }
     }
 }
 
@@ -1433,7 +1506,7 @@ __global__ void __launch_bounds__(256) copy_out_kernel(OutArgs a) {
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step) {
         Pack<T, V> v = ld_ro<T, V>(state + r * a.ld_state + c);
         apply_bias<T, V>(a, r, c, v);
-        st_pack(out + r * a.ld_out + c, v);
+        st_io(out + r * a.ld_out, c, a.k, a.vec, v);
     }
 }
 
@@ -1454,7 +1527,7 @@ __global__ void __launch_bounds__(256) emit_all_kernel(OutArgs a) {
     T* out = static_cast<T*>(a.out);
     const int64_t step = static_cast<int64_t>(V) << a.log2g;
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step)
-        st_pack(out + j * a.ld_out + c, ld_ro<T, V>(state + n * a.ld_state + c));
+        st_io(out + j * a.ld_out, c, a.k, a.vec, ld_ro<T, V>(state + n * a.ld_state + c));
 }
 
 // Output kernels for mixed storage: decode to FP64, 4 columns per lane, columns >= k skipped.
@@ -1566,6 +1639,29 @@ Shape choose_shape(const grg_b200_traverse_args* a) {
     int log2g = 0;
     while ((1 << log2g) < cols && log2g < 5) ++log2g;
     return {vec, log2g};
+}
+
+// Shape of the seed and output kernels: the widest vector that the state rows hold whole; `vec`
+// says whether the input, output and init rows take it too.
+struct IoShape {
+    Shape shape;
+    bool vec;
+};
+
+IoShape choose_io_shape(const grg_b200_traverse_args* a) {
+    if (a->dtype == GRG_B200_MIXED) return {choose_shape(a), false};
+    const int esize = a->dtype == GRG_B200_F64 ? 8 : 4;
+    int vec = 16 / esize;
+    while (vec > 1 && (a->ld_state % vec != 0 || !aligned(a->state, vec * esize) || a->k <= vec / 2)) vec >>= 1;
+    const int64_t lds[] = {a->ld_input, a->ld_output, a->use_miss ? a->ld_miss : 0, a->ld_init};
+    const void* ptrs[] = {a->input, a->output, a->use_miss ? a->miss : nullptr, a->init_vector, a->init_matrix};
+    bool whole = a->k % vec == 0;
+    for (int64_t ld : lds) whole = whole && ld % vec == 0;
+    for (const void* p : ptrs) whole = whole && aligned(p, vec * esize);
+    const int64_t cols = (a->k + vec - 1) / vec;
+    int log2g = 0;
+    while ((1 << log2g) < cols && log2g < 5) ++log2g;
+    return {{vec, log2g}, whole};
 }
 
 dim3 grid_for(int64_t rows, int log2g, int threads) {
@@ -2092,7 +2188,9 @@ int launch_run(const grg_b200_traverse_args* a, const Shape& sh, const LevelArgs
     return dispatch(a, sh, [&](auto t, auto v) { return launch_run_typed<decltype(t), decltype(v)::value>(p, a->init_mode, max_blocks, s); });
 }
 
-int seed_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
+int seed_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
+    const IoShape io = choose_io_shape(a);
+    const Shape& sh = io.shape;
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (a->level0_rows <= 0) return GRG_B200_OK;
     if (!a->input) return grg_fail(GRG_B200_ERR_INVALID, "input is NULL");
@@ -2110,17 +2208,17 @@ int seed_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t 
         using T = decltype(t);
         constexpr int V = decltype(v)::value;
         switch (a->init_mode) {
-            case 0: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 0>, la, a->num_samples, a->sample_to_individual, a->by_individual)); break;
-            case 1: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 1>, la, a->num_samples, a->sample_to_individual, a->by_individual)); break;
-            case 2: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 2>, la, a->num_samples, a->sample_to_individual, a->by_individual)); break;
-            default: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 3>, la, a->num_samples, a->sample_to_individual, a->by_individual)); break;
+            case 0: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 0>, la, io.vec, a->num_samples, a->sample_to_individual, a->by_individual)); break;
+            case 1: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 1>, la, io.vec, a->num_samples, a->sample_to_individual, a->by_individual)); break;
+            case 2: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 2>, la, io.vec, a->num_samples, a->sample_to_individual, a->by_individual)); break;
+            default: GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_kernel<T, V, 3>, la, io.vec, a->num_samples, a->sample_to_individual, a->by_individual)); break;
         }
         GRG_LAUNCH_CHECK("seed_up_kernel");
         return (int)GRG_B200_OK;
     });
 }
 
-OutArgs out_args(const grg_b200_traverse_args* a, const Shape& sh) {
+OutArgs out_args(const grg_b200_traverse_args* a, const IoShape& io) {
     OutArgs o{};
     o.state = a->state;
     o.ld_state = a->ld_state;
@@ -2130,7 +2228,8 @@ OutArgs out_args(const grg_b200_traverse_args* a, const Shape& sh) {
     o.init_vector = a->init_vector;
     o.bias_mode = a->emit_all_nodes ? GRG_B200_BIAS_NONE : a->bias_mode;
     o.k = a->k;
-    o.log2g = sh.log2g;
+    o.log2g = io.shape.log2g;
+    o.vec = io.vec;
     o.err = a->error_word;
     o.lim = a->num_nodes;
     if (a->dtype == GRG_B200_MIXED)
@@ -2138,13 +2237,22 @@ OutArgs out_args(const grg_b200_traverse_args* a, const Shape& sh) {
     return o;
 }
 
-int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
+template <typename T, int V, bool BIAS_PER_ENTRY>
+cudaError_t launch_gather_out(bool pdl, cudaStream_t s, const OutArgs& o) {
+    if ((o.rows << o.log2g) <= int64_t{148} * 2048)
+        return launch_k(pdl, s, grid_for(o.rows, o.log2g, 256), 256, gather_out_kernel<T, V, BIAS_PER_ENTRY, 1>, o);
+    return launch_k(pdl, s, grid_for((o.rows + kOutRows - 1) / kOutRows, o.log2g, 256), 256, gather_out_kernel<T, V, BIAS_PER_ENTRY, kOutRows>, o);
+}
+
+int output_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
+    const IoShape io = choose_io_shape(a);
+    const Shape& sh = io.shape;
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (!a->output || !a->sel_mut_ptr || (!a->sel_mut_idx && a->num_mutations > 0))
         return grg_fail(GRG_B200_ERR_INVALID, "up output needs output and sel_mut");
     if (a->use_miss && (!a->miss || !a->sel_miss_ptr)) return grg_fail(GRG_B200_ERR_INVALID, "up miss output needs miss and sel_miss");
     if (a->num_mutations == 0) return GRG_B200_OK;
-    OutArgs o = out_args(a, sh);
+    OutArgs o = out_args(a, io);
     o.rows = a->num_mutations;
     o.ptr = a->sel_mut_ptr;
     o.idx = a->sel_mut_idx;
@@ -2167,7 +2275,7 @@ int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_
     return dispatch(a, sh, [&](auto t, auto v) {
         using T = decltype(t);
         constexpr int V = decltype(v)::value;
-        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_kernel<T, V, false>, o));
+        GRG_CUDA_TRY(launch_gather_out<T, V, false>(pdl, s, o));
         GRG_LAUNCH_CHECK("gather_out_kernel(sel_mut)");
         if (a->use_miss) {
             OutArgs m = o;
@@ -2176,17 +2284,19 @@ int output_up_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_
             m.out = a->miss;
             m.ld_out = a->ld_miss;
             m.bias_mode = GRG_B200_BIAS_NONE;
-            GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_kernel<T, V, false>, m));
+            GRG_CUDA_TRY(launch_gather_out<T, V, false>(pdl, s, m));
             GRG_LAUNCH_CHECK("gather_out_kernel(sel_miss)");
         }
         return (int)GRG_B200_OK;
     });
 }
 
-int output_down_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
+int output_down_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
+    const IoShape io = choose_io_shape(a);
+    const Shape& sh = io.shape;
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (!a->output) return grg_fail(GRG_B200_ERR_INVALID, "output is NULL");
-    OutArgs o = out_args(a, sh);
+    OutArgs o = out_args(a, io);
     if (a->by_individual) {
         if (!a->ind_ptr || !a->ind_samples) return grg_fail(GRG_B200_ERR_INVALID, "by_individual needs ind_ptr/ind_samples");
         o.rows = a->num_individuals;
@@ -2207,17 +2317,19 @@ int output_down_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStrea
     return dispatch(a, sh, [&](auto t, auto v) {
         using T = decltype(t);
         constexpr int V = decltype(v)::value;
-        if (a->by_individual) GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_kernel<T, V, true>, o));
+        if (a->by_individual) GRG_CUDA_TRY(launch_gather_out<T, V, true>(pdl, s, o));
         else GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, copy_out_kernel<T, V>, o));
         GRG_LAUNCH_CHECK("output_down");
         return (int)GRG_B200_OK;
     });
 }
 
-int emit_all_impl(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t s) {
+int emit_all_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
+    const IoShape io = choose_io_shape(a);
+    const Shape& sh = io.shape;
     const bool pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
     if (!a->output || !a->inv_node_perm) return grg_fail(GRG_B200_ERR_INVALID, "emit_all_nodes needs output and inv_node_perm");
-    OutArgs o = out_args(a, sh);
+    OutArgs o = out_args(a, io);
     o.rows = a->num_nodes;
     o.idx = a->inv_node_perm;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
@@ -2311,7 +2423,7 @@ int run_dataflow(const grg_b200_traverse_args* a, const Shape& sh, cudaStream_t 
         GRG_LAUNCH_CHECK("sentinel_fill_kernel");
     }
     if (a->direction == GRG_B200_UP) {
-        const int rc = seed_up_impl(a, sh, s);
+        const int rc = seed_up_impl(a, s);
         if (rc) return rc;
     }
     if (tasks == 0) return GRG_B200_OK;
@@ -2550,7 +2662,7 @@ int grg_b200_ring_destroy(grg_b200_ring* r) {
 int grg_b200_seed_up(const grg_b200_traverse_args* a, void* stream) {
     int rc = validate_common(a);
     if (rc) return rc;
-    return seed_up_impl(a, choose_shape(a), static_cast<cudaStream_t>(stream));
+    return seed_up_impl(a, static_cast<cudaStream_t>(stream));
 }
 
 int grg_b200_run_level(const grg_b200_traverse_args* a, const grg_b200_level* level, void* stream) {
@@ -2563,19 +2675,19 @@ int grg_b200_run_level(const grg_b200_traverse_args* a, const grg_b200_level* le
 int grg_b200_output_up(const grg_b200_traverse_args* a, void* stream) {
     int rc = validate_common(a);
     if (rc) return rc;
-    return output_up_impl(a, choose_shape(a), static_cast<cudaStream_t>(stream));
+    return output_up_impl(a, static_cast<cudaStream_t>(stream));
 }
 
 int grg_b200_output_down(const grg_b200_traverse_args* a, void* stream) {
     int rc = validate_common(a);
     if (rc) return rc;
-    return output_down_impl(a, choose_shape(a), static_cast<cudaStream_t>(stream));
+    return output_down_impl(a, static_cast<cudaStream_t>(stream));
 }
 
 int grg_b200_emit_all(const grg_b200_traverse_args* a, void* stream) {
     int rc = validate_common(a);
     if (rc) return rc;
-    return emit_all_impl(a, choose_shape(a), static_cast<cudaStream_t>(stream));
+    return emit_all_impl(a, static_cast<cudaStream_t>(stream));
 }
 
 int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
@@ -2603,9 +2715,9 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
     if (!any_streamed && dataflow_eligible(a)) {
         rc = run_dataflow(a, sh, s);
         if (rc) return rc;
-        if (a->emit_all_nodes) return emit_all_impl(a, sh, s);
-        if (a->direction == GRG_B200_UP) return output_up_impl(a, sh, s);
-        return output_down_impl(a, sh, s);
+        if (a->emit_all_nodes) return emit_all_impl(a, s);
+        if (a->direction == GRG_B200_UP) return output_up_impl(a, s);
+        return output_down_impl(a, s);
     }
     grg_b200_traverse_args no_pdl;
     if (any_streamed && (a->launch_flags & GRG_B200_LAUNCH_PDL)) {  // ring copies sit between the level launches
@@ -2614,7 +2726,7 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
         a = &no_pdl;
     }
     if (a->direction == GRG_B200_UP) {
-        rc = seed_up_impl(a, sh, s);
+        rc = seed_up_impl(a, s);
         if (rc) return rc;
     } else if (a->dtype == GRG_B200_MIXED) {
         rc = encode_down_inputs(a, sh, s);
@@ -2669,9 +2781,9 @@ int grg_b200_traverse(const grg_b200_traverse_args* a, void* stream_handle) {
         GRG_CUDA_TRY(cudaEventRecord(a->ring->join, a->ring->copy));
         GRG_CUDA_TRY(cudaStreamWaitEvent(s, a->ring->join, 0));
     }
-    if (a->emit_all_nodes) return emit_all_impl(a, sh, s);
-    if (a->direction == GRG_B200_UP) return output_up_impl(a, sh, s);
-    return output_down_impl(a, sh, s);
+    if (a->emit_all_nodes) return emit_all_impl(a, s);
+    if (a->direction == GRG_B200_UP) return output_up_impl(a, s);
+    return output_down_impl(a, s);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -2831,7 +2943,12 @@ int grg_b200_traverse_static(const grg_b200_traverse_args* a, void* stream_handl
     if (rc) return rc;
     grg_b200_traverse_args local = *a;
     local.state = state;
-    local.ld_state = a->k;
+    // rows of whole vectors, as grg_b200_traverse's caller would lay them out, where they fit
+    const int64_t chunk = 32 / esize;
+    int64_t padded = 1;
+    while (padded < a->k && padded < chunk) padded <<= 1;
+    if (a->k > chunk) padded = (a->k + chunk - 1) / chunk * chunk;
+    local.ld_state = a->num_nodes <= (int64_t)GRG_B200_STATIC_STATE_BYTES / esize / padded ? padded : a->k;
     local.ring = nullptr;
     local.slot_buffers = nullptr;
     local.slot_bytes = nullptr;

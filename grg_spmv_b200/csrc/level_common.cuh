@@ -15,11 +15,11 @@ __attribute__((visibility("hidden"))) int grg_fail(int code, const char* fmt, ..
 
 namespace grg {
 
-#define GRG_CUDA_TRY(expr)                                                                  \
+#define GRG_CUDA_TRY(...)                                                                   \
     do {                                                                                    \
-        cudaError_t err__ = (expr);                                                         \
+        cudaError_t err__ = (__VA_ARGS__);                                                       \
         if (err__ != cudaSuccess)                                                           \
-            return grg_fail(GRG_B200_ERR_CUDA, "%s failed: %s", #expr, cudaGetErrorString(err__)); \
+            return grg_fail(GRG_B200_ERR_CUDA, "%s failed: %s", #__VA_ARGS__, cudaGetErrorString(err__)); \
     } while (0)
 
 #define GRG_LAUNCH_CHECK(name)                                                              \

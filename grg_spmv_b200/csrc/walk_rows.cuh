@@ -309,7 +309,10 @@ int launch_rows(const LevelArgs& la, int init_mode, int64_t num_entries, const i
     //   1.5M nodes up k = 1: 250 / 207 / 160, k = 8: 382 / 242 / 267, k = 32: 517 / 549 / 791;
     //   5M nodes up k = 1: 419 / 303 / 371, k = 8: 617 / 617 / 802, k = 16: 945 / 1015 / 1407.
     ws.slots = 4;
-    while (ws.slots > 1 && (ws.w * ws.slots > 32 || (long_rows * ws.slots + la.short_rows) * ws.w > 32 * kSlotWarps)) ws.slots >>= 1;
+    const auto level_warps = [&](int slots) {
+        return (long_rows + 32 / (ws.w * slots) - 1) / (32 / (ws.w * slots)) + (la.short_rows + ws.short_rows_per_warp - 1) / ws.short_rows_per_warp;
+    };
+    while (ws.slots > 1 && (ws.w * ws.slots > 32 || level_warps(ws.slots) > kSlotWarps)) ws.slots >>= 1;
     ws.inv_group = inverse16(ws.w * ws.slots);
     ws.rows_per_warp = 32 / (ws.w * ws.slots);
     const bool only_heavy = narrow == 0;
