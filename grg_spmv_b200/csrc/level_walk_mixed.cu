@@ -1,7 +1,7 @@
 // The row walk over mixed storage (GRG_B200_MIXED, mixed.cuh): the kernels of walk_rows.cuh with
 // rows of 6-byte values, FP64 sums, and any init.
 //
-// The walk is bound by instruction issue: a value costs five integer instructions (the words moved
+// The walk is bound by instruction issue: a value costs four or five integer instructions (the words moved
 // into a double's place), one FP32 fma (the test for infinities and NaN) and one FP64 fma, where the
 // earlier format (a signed correction to a rounded FP32 value) took two conversions, the unit of
 // the correction and a test, in kernels with per-segment sums and a second launch for heavy rows.
@@ -94,8 +94,8 @@ struct MixedRows {
 #pragma unroll
                 for (int i = 0; i < kMxCols; i += 2) {
                     const uint32_t l = r[u].lo[i / 2];
-                    acc.v[i] = __fma_rn(mx_scaled(r[u].hi[i], (l << 13) & 0x1fffe000u), up, acc.v[i]);
-                    acc.v[i + 1] = __fma_rn(mx_scaled(r[u].hi[i + 1], (l >> 3) & 0x1fffe000u), up, acc.v[i + 1]);
+                    acc.v[i] = __fma_rn(mx_scaled<UPONLY>(r[u].hi[i], UPONLY ? l << 16 : (l << 13) & 0x1fffe000u), up, acc.v[i]);
+                    acc.v[i + 1] = __fma_rn(mx_scaled<UPONLY>(r[u].hi[i + 1], UPONLY ? l & 0xffff0000u : (l >> 3) & 0x1fffe000u), up, acc.v[i + 1]);
                 }
         } else {
 #pragma unroll
