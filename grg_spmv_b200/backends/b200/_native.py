@@ -34,6 +34,7 @@ LAUNCH_PDL = 1
 LAUNCH_WALK = 2
 LONG_ROW = 512
 LONG_CLASSES = 8
+QUAD_CLASSES = 8
 SCHEDULE_LEVELS, SCHEDULE_DATAFLOW = 0, 1
 DEVICE_WAIT_TIMEOUT = 6
 UP, DOWN = 0, 1
@@ -85,6 +86,7 @@ class Level(ctypes.Structure):
         ("slot_width", ctypes.c_int32 * 8),
         ("short_rows", ctypes.c_int64),
         ("long_rows", ctypes.c_int64 * LONG_CLASSES),
+        ("quad_rows", ctypes.c_int64 * QUAD_CLASSES),
     ]
 
 

@@ -93,6 +93,18 @@ class LevelGather:
         longer = np.flatnonzero(np.diff(self.row_ptr[:narrow + 1].astype(np.int64)) > 4)
         return narrow - (int(longer[-1]) + 1 if longer.size else 0)
 
+    def quad_rows(self) -> list[int]:
+        """How many narrow positions hold more than i quads, for i up to ``QUAD_CLASSES``, where the
+        narrow positions are in descending order of quads (the default long-first order of padded
+        lists) and none holds more; else zeros.  Kernels locate such lists by arithmetic."""
+        narrow = self.num_rows - int(self.heavy_rows.size)
+        if self.list_align != 4 or narrow <= 0:
+            return [0] * nat.QUAD_CLASSES
+        quads = np.diff(self.row_ptr[:narrow + 1]) >> 2
+        if int(quads[0]) > nat.QUAD_CLASSES or np.any(quads[1:] > quads[:-1]):
+            return [0] * nat.QUAD_CLASSES
+        return (narrow - np.searchsorted(quads[::-1], np.arange(nat.QUAD_CLASSES), side="right")).tolist()
+
     def long_rows(self) -> list[int]:
         """How many heavy rows hold more than ``LONG_ROW << i`` entries: the first so many of
         ``heavy_rows``, which kernels may split further than the others."""
@@ -167,7 +179,8 @@ _LONG = np.asarray([nat.LONG_ROW << i for i in range(nat.LONG_CLASSES)], dtype=n
 
 def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np.ndarray, src: np.ndarray,
             group: np.ndarray, heavy_threshold: int, locality: bool = False, balance: bool = True,
-            pad: bool = False, long_first: bool = True, slots: bool = False, heavy_buckets: bool = False) -> LevelGather:
+            pad: bool = False, long_first: bool = True, slots: bool = False, heavy_buckets: bool = False,
+            quad_order: bool = True) -> LevelGather:
     """Stable-sort the concatenated pieces by row, flag segment starts, build row_ptr.
 
     With ``locality`` the rows are stored in the order of the id of their last state entry
@@ -188,9 +201,9 @@ def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np
         start[1:] = (rows[1:] != rows[:-1]) | (group[1:] != group[:-1])
     entries = (ids.astype(np.uint32) | (src.astype(np.uint32) << np.uint32(nat.SRC_SHIFT))
                | np.where(start, np.uint32(nat.SEG_START), np.uint32(0))).astype(np.uint32)
-    # Processing order: narrow rows first, grouped into power-of-two length buckets so the rows
-    # of a warp need similar trip counts (in locality order inside a bucket when asked), the
-    # longest bucket first (``long_first``: CTAs start in index order, so the longest chains of
+    # Processing order: narrow rows first, grouped into length buckets (powers of two; by quads as
+    # well for padded lists, longest first) so the rows of a warp need similar trip counts (in
+    # locality order inside a bucket when asked), the longest bucket first (``long_first``: CTAs start in index order, so the longest chains of
     # dependent loads start earliest and short rows fill in behind them); heavy rows last.
     perm = np.arange(num_rows, dtype=np.int64)
     if locality and num_rows > 1:
@@ -210,6 +223,8 @@ def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np
             bucket = _quad_class(counts[narrow_perm])
         else:
             bucket = _bit_length(counts[narrow_perm])
+            if quad_order and pad and long_first:  # equal quads together: every row of a warp takes the same rounds
+                bucket += 64 * ((counts[narrow_perm] + 3) // 4)
         narrow_perm = narrow_perm[_stable_argsort(-bucket if long_first else bucket)]
     if balance and heavy_buckets and heavy_perm.size > 1:
         bucket = _bit_length(counts[heavy_perm])
@@ -257,7 +272,7 @@ def _finish(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np
 def _finish_torch(level: int, row_begin: int, num_rows: int, rows: np.ndarray, ids: np.ndarray, src: np.ndarray,
                   group: np.ndarray, heavy_threshold: int, locality: bool = False, balance: bool = True,
                   pad: bool = False, long_first: bool = True, slots: bool = False, heavy_buckets: bool = False,
-                  device="cuda") -> LevelGather:
+                  quad_order: bool = True, device="cuda") -> LevelGather:
     """``_finish`` with PyTorch on ``device`` (the GPU when the runtime builds its levels):
     the same steps as the NumPy version, in integer arithmetic only, so the lists, row
     pointers, processing order and slot tables are identical to it."""
@@ -310,6 +325,8 @@ def _finish_torch(level: int, row_begin: int, num_rows: int, rows: np.ndarray, i
     if balance and narrow_perm.numel() > 1:
         c = counts[narrow_perm]
         bucket = quad_class(c) if use_slots else torch.searchsorted(pow2, c, right=True)
+        if quad_order and pad and long_first and not use_slots:
+            bucket = bucket + 64 * ((c + 3) // 4)
         narrow_perm = narrow_perm[torch.sort(-bucket if long_first else bucket, stable=True).indices]
     if balance and heavy_buckets and heavy_perm.numel() > 1:
         bucket = torch.searchsorted(pow2, counts[heavy_perm], right=True)
@@ -373,9 +390,13 @@ def load_blocks(blocks) -> dict[tuple[int, int], tuple[np.ndarray, np.ndarray]]:
 
 def build_up_levels(level_offsets: np.ndarray, coo: dict, heavy_threshold: int, locality: bool = False,
                     balance: bool = True, pad: bool = False, long_first: bool = True, slots: bool = False,
-                    device=None, heavy_buckets: bool = False) -> list[LevelGather]:
+                    device=None, heavy_buckets: bool = False, quad_order: bool = True) -> list[LevelGather]:
     """Gather lists for up levels 1..h-1 (level 0 is seeded from the input); built with
-    PyTorch on ``device`` when given (identical results), else with NumPy."""
+    PyTorch on ``device`` when given (identical results), else with NumPy.
+
+    ``quad_order``: padded narrow rows of equal quads together, not only of one power of two: the
+    rows of a warp take the same rounds, and kernels find their lists without row pointers
+    (``LevelGather.quad_rows``)."""
     finish = _finish if device is None else (lambda *a: _finish_torch(*a, device=device))
     off = np.asarray(level_offsets, dtype=np.int64)
     h = off.size - 1
@@ -392,7 +413,7 @@ def build_up_levels(level_offsets: np.ndarray, coo: dict, heavy_threshold: int, 
             src.append(np.full(r.size, s, dtype=np.int16))
         cat = (lambda parts, dt: np.concatenate(parts) if parts else np.empty(0, dtype=dt))
         r, i, g = cat(rows, np.int64), cat(ids, np.int64), cat(src, np.int16)
-        levels.append(finish(dst, int(off[dst]), n, r, i, np.zeros(i.size, np.uint8), g, heavy_threshold, locality, balance, pad, long_first, slots, heavy_buckets))
+        levels.append(finish(dst, int(off[dst]), n, r, i, np.zeros(i.size, np.uint8), g, heavy_threshold, locality, balance, pad, long_first, slots, heavy_buckets, quad_order))
     return levels
 
 
@@ -408,7 +429,7 @@ def _selector_by_node(ptr: np.ndarray, idx: np.ndarray, num_rows: int) -> tuple[
 def build_down_levels(level_offsets: np.ndarray, coo: dict, sel_mut, sel_miss, heavy_threshold: int,
                       locality: bool = True, balance: bool = True, pad: bool = False,
                       long_first: bool = True, slots: bool = False, device=None,
-                      heavy_buckets: bool = False) -> list[LevelGather]:
+                      heavy_buckets: bool = False, quad_order: bool = True) -> list[LevelGather]:
     """Gather lists for down levels h-1..0 in execution order (PyTorch on ``device`` when
     given, identical results).
 
@@ -445,7 +466,7 @@ def build_down_levels(level_offsets: np.ndarray, coo: dict, sel_mut, sel_miss, h
         cat = (lambda parts, dt: np.concatenate(parts) if parts else np.empty(0, dtype=dt))
         levels.append(finish(dst, lo, hi - lo, cat(rows, np.int64), cat(ids, np.int64), cat(src, np.uint8),
                               cat(grp, np.int16), heavy_threshold, locality, balance, pad, long_first, slots,
-                              heavy_buckets))
+                              heavy_buckets, quad_order))
     return levels
 
 

@@ -2061,6 +2061,15 @@ int build_level_args(const grg_b200_traverse_args* a, const Shape& sh, const grg
         return grg_fail(GRG_B200_ERR_INVALID, "short_rows %lld outside [0, %lld]", (long long)L->short_rows,
                     (long long)(L->num_rows - L->num_heavy));
     la.short_rows = L->short_rows;
+    int64_t quads = 0;
+    for (int i = 0; i < GRG_B200_QUAD_CLASSES; ++i) {
+        quads += L->quad_rows[i];
+        if (L->quad_rows[i] < 0 || L->quad_rows[i] > (i ? L->quad_rows[i - 1] : L->num_rows - L->num_heavy) || L->quad_rows[i] > INT32_MAX)
+            return grg_fail(GRG_B200_ERR_INVALID, "quad_rows[%d] %lld is out of order or above the narrow rows", i, (long long)L->quad_rows[i]);
+        la.quad_rows[i] = static_cast<int32_t>(L->quad_rows[i]);
+    }
+    if (quads * 4 > L->num_entries || (quads > 0 && L->list_align != 4))
+        return grg_fail(GRG_B200_ERR_INVALID, "quad_rows name %lld quads, the level has %lld entries", (long long)quads, (long long)L->num_entries);
     la.num_slot_buckets = 0;
     if (L->num_slot_buckets < 0 || L->num_slot_buckets > GRG_B200_MAX_SLOT_BUCKETS)
         return grg_fail(GRG_B200_ERR_INVALID, "num_slot_buckets %d outside [0, %d]", L->num_slot_buckets, GRG_B200_MAX_SLOT_BUCKETS);

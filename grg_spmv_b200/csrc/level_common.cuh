@@ -190,6 +190,7 @@ struct LevelArgs {
     const void* miss_lo;
     int32_t up;  // an up level: its lists name state rows (and null padding) only
     int64_t short_rows;  // entry kernels: the last short_rows narrow positions take one entry slot
+    int32_t quad_rows[GRG_B200_QUAD_CLASSES];  // row walk: narrow positions of more than i quads; [0] = 0: read row_ptr
 };
 
 enum DeviceError : int32_t {

@@ -80,6 +80,25 @@ __device__ __forceinline__ SlotCodes<S> null_codes() {
     return r;
 }
 
+// The quads [q0, q1) of a narrow position: by arithmetic where the level's rows are in order of their
+// quads, which takes the row pointers' latency off every CTA's way to its first fetch.
+__device__ __forceinline__ void narrow_quads(const LevelArgs& a, int64_t pos, int32_t& q0, int32_t& q1) {
+    if (a.quad_rows[0] > 0) {
+        const int32_t p = static_cast<int32_t>(pos);
+        q0 = 0;
+        int32_t n = 0;
+#pragma unroll
+        for (int i = 0; i < GRG_B200_QUAD_CLASSES; ++i) {
+            q0 += min(p, a.quad_rows[i]);
+            n += p < a.quad_rows[i];
+        }
+        q1 = q0 + n;
+    } else {
+        q0 = __ldg(a.row_ptr + pos) >> 2;
+        q1 = __ldg(a.row_ptr + pos + 1) >> 2;
+    }
+}
+
 // Narrow rows with S entry slots.  The list is static, so its extent and the codes of its first
 // 2 S quads (8 codes a lane) are loaded before the wait on the previous level.
 template <class R, int NW, int S, int LB>
@@ -102,8 +121,7 @@ __device__ __forceinline__ void walk_rows(const LevelArgs& a, const WalkShape& w
 #pragma unroll
     for (int j = 0; j < PQ; ++j) pre[j] = null_codes<S>();
     if (live) {
-        q0 = __ldg(a.row_ptr + pos) >> 2;
-        q1 = __ldg(a.row_ptr + pos + 1) >> 2;
+        narrow_quads(a, pos, q0, q1);
         row = level_row(a, pos);
 #pragma unroll
         for (int j = 0; j < PQ; ++j)

@@ -130,6 +130,7 @@ typedef enum grg_b200_bias {
 /* Very long rows: class i holds the rows of more than GRG_B200_LONG_ROW << i entries. */
 #define GRG_B200_LONG_ROW 512
 #define GRG_B200_LONG_CLASSES 8
+#define GRG_B200_QUAD_CLASSES 8 /* narrow lists of up to 8 quads can be located without row_ptr */
 
 typedef struct grg_b200_level {
     int64_t row_begin;
@@ -158,6 +159,11 @@ typedef struct grg_b200_level {
                            than GRG_B200_LONG_ROW << i entries; heavy_rows lists them first, longest
                            class first, so they are its first long_rows[i] members.  0 for all when
                            heavy_rows is in another order. */
+    int64_t quad_rows[GRG_B200_QUAD_CLASSES]; /* quad_rows[i]: how many of the narrow positions hold
+                           more than i quads (4 entries), where the narrow positions are in order of
+                           their quads, most first, and none holds more than GRG_B200_QUAD_CLASSES.  A
+                           position's list then starts after sum(min(position, quad_rows[i]))
+                           quads, and row_ptr need not be read.  0 for all otherwise. */
 } grg_b200_level;
 
 typedef struct grg_b200_ring grg_b200_ring; /* opaque: copy stream + per-slot events */
