@@ -989,18 +989,20 @@ __global__ void __launch_bounds__(kNarrowThreads, MB) level_run_kernel(const __g
 // columns (ld % 4 == 0) is two planes: uint32 hi[R * ld] followed by uint16 lo[R * ld].
 // ---------------------------------------------------------------------------------------
 // Encoded copy of an FP64 matrix: dst[r, c] = src[r, c] for c < k, 0 for k <= c < ld.
-__global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, int64_t ld_src, int64_t rows, int64_t k,
+__global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, int64_t ld_src, int64_t rows, int64_t k, bool vec,
                                                              uint32_t* dst_hi, uint16_t* dst_lo, int64_t ld, int32_t log2g) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t r = t >> log2g;
     if (r >= rows) return;
     const int lane = static_cast<int>(t & ((1 << log2g) - 1));
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < ld; c += static_cast<int64_t>(4) << log2g)
-        mx_store(dst_hi + r * ld + c, dst_lo + r * ld + c, f64_load_guarded(src + r * ld_src, c, k));
+        mx_store(dst_hi + r * ld + c, dst_lo + r * ld + c, f64_load(src + r * ld_src, c, k, vec));
 }
 
 // Up seeding of level 0 in mixed storage: state[r] = init(r) (+ input row for samples).
-__global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, int init_mode, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
+__global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, bool vec, int init_mode, int64_t num_samples, const int32_t* s2i, int32_t by_ind) {
     pdl_trigger();
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t row = t >> a.log2g;
@@ -1017,7 +1019,7 @@ __global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, int init_m
     const double* x = static_cast<const double*>(a.x);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
         Quad v = mx_init(a, init_mode, row, c);
-        if (row < num_samples) add_quad(v, f64_load_guarded(x + xrow * a.ld_x, c, a.k));
+        if (row < num_samples) add_quad(v, f64_load(x + xrow * a.ld_x, c, a.k, vec));
         const int64_t o = row * a.ld_state + c;
         mx_store(static_cast<uint32_t*>(a.state) + o, static_cast<uint16_t*>(a.state_lo) + o, v);
     }
@@ -1538,7 +1540,7 @@ __device__ __forceinline__ void mx_apply_bias(const OutArgs& a, int64_t r, int64
         for (int i = 0; i < 4; ++i) v.v[i] = __dadd_rn(v.v[i], b);
     } else if (a.bias_mode == GRG_B200_BIAS_VECTOR) {
         const double b = __ldg(static_cast<const double*>(a.bias) + r);
-        const Quad iv = f64_load_guarded(static_cast<const double*>(a.init_vector), c, a.k);
+        const Quad iv = f64_load(static_cast<const double*>(a.init_vector), c, a.k, false);
 #pragma unroll
         for (int i = 0; i < 4; ++i) v.v[i] = __dadd_rn(v.v[i], __dmul_rn(b, iv.v[i]));
     }
@@ -1549,29 +1551,55 @@ __device__ __forceinline__ Quad mx_state_row(const OutArgs& a, int64_t n, int64_
     return mx_load(static_cast<const uint32_t*>(a.state) + o, static_cast<const uint16_t*>(a.state_lo) + o);
 }
 
-template <bool BIAS_PER_ENTRY>
+// As gather_out_kernel: R rows per lane group, their extents and first indexes loaded before the
+// wait and their first state rows in flight together.
+template <bool BIAS_PER_ENTRY, int R>
 __global__ void __launch_bounds__(256) gather_out_mx_kernel(OutArgs a) {
+    const int per_block = 256 >> a.log2g;
+    const int lane = static_cast<int>(threadIdx.x) & ((1 << a.log2g) - 1);
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * per_block * R + (threadIdx.x >> a.log2g);
+    int32_t e0[R], e1[R];
+    int64_t n0[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const int64_t r = first + static_cast<int64_t>(u) * per_block;
+        e0[u] = r < a.rows ? __ldg(a.ptr + r) : 0;
+        e1[u] = r < a.rows ? __ldg(a.ptr + r + 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) n0[u] = e0[u] < e1[u] ? __ldg(a.idx + e0[u]) : 0;
     pdl_wait();
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t r = t >> a.log2g;
-    if (r >= a.rows) return;
-    const int lane = static_cast<int>(t & ((1 << a.log2g) - 1));
-    const int32_t e0 = __ldg(a.ptr + r), e1 = __ldg(a.ptr + r + 1);
     double* out = static_cast<double*>(a.out);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
-        Quad s = zero_quad();
-        for (int32_t e = e0; e < e1; ++e) {
-            const int64_t n = __ldg(a.idx + e);
-            if (a.err && (n < 0 || n >= a.lim)) {
-                report(a.err, kErrSelector);
-                continue;
+        Quad v[R];
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            v[u] = zero_quad();
+            if (e0[u] < e1[u]) {
+                if (a.err && (n0[u] < 0 || n0[u] >= a.lim)) report(a.err, kErrSelector);
+                else v[u] = mx_state_row(a, n0[u], c);
             }
-            Quad v = mx_state_row(a, n, c);
-            if constexpr (BIAS_PER_ENTRY) mx_apply_bias(a, n, c, v);
-            add_quad(s, v);
         }
-        if constexpr (!BIAS_PER_ENTRY) mx_apply_bias(a, r, c, s);
-        f64_store_guarded(out + r * a.ld_out, c, a.k, s);
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int64_t r = first + static_cast<int64_t>(u) * per_block;
+            if (r < a.rows) {
+                Quad s = zero_quad();
+                for (int32_t e = e0[u]; e < e1[u]; ++e) {
+                    int64_t n = n0[u];
+                    if (e > e0[u]) n = __ldg(a.idx + e);
+                    if (a.err && (n < 0 || n >= a.lim)) {
+                        report(a.err, kErrSelector);
+                        continue;
+                    }
+                    if (e > e0[u]) v[u] = mx_state_row(a, n, c);
+                    if constexpr (BIAS_PER_ENTRY) mx_apply_bias(a, n, c, v[u]);
+                    add_quad(s, v[u]);
+                }
+                if constexpr (!BIAS_PER_ENTRY) mx_apply_bias(a, r, c, s);
+                f64_store(out + r * a.ld_out, c, a.k, a.vec, s);
+            }
+        }
     }
 }
 
@@ -1585,7 +1613,7 @@ __global__ void __launch_bounds__(256) copy_out_mx_kernel(OutArgs a) {
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
         Quad v = mx_state_row(a, r, c);
         mx_apply_bias(a, r, c, v);
-        f64_store_guarded(out + r * a.ld_out, c, a.k, v);
+        f64_store(out + r * a.ld_out, c, a.k, a.vec, v);
     }
 }
 
@@ -1602,7 +1630,7 @@ __global__ void __launch_bounds__(256) emit_all_mx_kernel(OutArgs a) {
     }
     double* out = static_cast<double*>(a.out);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g)
-        f64_store_guarded(out + j * a.ld_out, c, a.k, mx_state_row(a, n, c));
+        f64_store(out + j * a.ld_out, c, a.k, a.vec, mx_state_row(a, n, c));
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1649,7 +1677,13 @@ struct IoShape {
 };
 
 IoShape choose_io_shape(const grg_b200_traverse_args* a) {
-    if (a->dtype == GRG_B200_MIXED) return {choose_shape(a), false};
+    if (a->dtype == GRG_B200_MIXED) {  // 4 columns a lane; FP64 rows in 16-byte accesses
+        bool whole = a->k % 4 == 0;
+        for (int64_t ld : {a->ld_input, a->ld_output, a->use_miss ? a->ld_miss : int64_t{0}}) whole = whole && ld % 2 == 0;
+        for (const void* p : {a->input, static_cast<const void*>(a->output), a->use_miss ? static_cast<const void*>(a->miss) : nullptr})
+            whole = whole && aligned(p, 16);
+        return {choose_shape(a), whole};
+    }
     const int esize = a->dtype == GRG_B200_F64 ? 8 : 4;
     int vec = 16 / esize;
     while (vec > 1 && (a->ld_state % vec != 0 || !aligned(a->state, vec * esize) || a->k <= vec / 2)) vec >>= 1;
@@ -2209,7 +2243,7 @@ int seed_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
     la.num_rows = a->level0_rows;
     const dim3 grid = grid_for(la.num_rows, la.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_mx_kernel, la, a->init_mode, a->num_samples, a->sample_to_individual, a->by_individual));
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, seed_up_mx_kernel, la, io.vec, a->init_mode, a->num_samples, a->sample_to_individual, a->by_individual));
         GRG_LAUNCH_CHECK("seed_up_mx_kernel");
         return (int)GRG_B200_OK;
     }
@@ -2246,6 +2280,13 @@ OutArgs out_args(const grg_b200_traverse_args* a, const IoShape& io) {
     return o;
 }
 
+template <bool BIAS_PER_ENTRY>
+cudaError_t launch_gather_out_mx(bool pdl, cudaStream_t s, const OutArgs& o) {
+    if ((o.rows << o.log2g) <= int64_t{148} * 2048)
+        return launch_k(pdl, s, grid_for(o.rows, o.log2g, 256), 256, gather_out_mx_kernel<BIAS_PER_ENTRY, 1>, o);
+    return launch_k(pdl, s, grid_for((o.rows + kOutRows - 1) / kOutRows, o.log2g, 256), 256, gather_out_mx_kernel<BIAS_PER_ENTRY, kOutRows>, o);
+}
+
 template <typename T, int V, bool BIAS_PER_ENTRY>
 cudaError_t launch_gather_out(bool pdl, cudaStream_t s, const OutArgs& o) {
     if ((o.rows << o.log2g) <= int64_t{148} * 2048)
@@ -2267,7 +2308,7 @@ int output_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
     o.idx = a->sel_mut_idx;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, o));
+        GRG_CUDA_TRY(launch_gather_out_mx<false>(pdl, s, o));
         GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_mut)");
         if (a->use_miss) {
             OutArgs m = o;
@@ -2276,7 +2317,7 @@ int output_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
             m.out = a->miss;
             m.ld_out = a->ld_miss;
             m.bias_mode = GRG_B200_BIAS_NONE;
-            GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, m));
+            GRG_CUDA_TRY(launch_gather_out_mx<false>(pdl, s, m));
             GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_miss)");
         }
         return (int)GRG_B200_OK;
@@ -2318,7 +2359,7 @@ int output_down_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
     if (o.rows == 0) return GRG_B200_OK;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        if (a->by_individual) GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<true>, o));
+        if (a->by_individual) GRG_CUDA_TRY(launch_gather_out_mx<true>(pdl, s, o));
         else GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, copy_out_mx_kernel, o));
         GRG_LAUNCH_CHECK("output_down_mx");
         return (int)GRG_B200_OK;
@@ -2447,14 +2488,13 @@ int encode_down_inputs(const grg_b200_traverse_args* a, const Shape& sh, cudaStr
     int log2g = 0;
     while ((1 << log2g) < (ld + 3) / 4 && log2g < 5) ++log2g;
     const dim3 grid = grid_for(a->num_mutations, log2g, 256);
-    mx_encode_rows_kernel<<<grid, 256, 0, s>>>(static_cast<const double*>(a->input), a->ld_input, a->num_mutations, a->k,
-                                               static_cast<uint32_t*>(const_cast<void*>(la.x)),
-                                               static_cast<uint16_t*>(const_cast<void*>(la.x_lo)), ld, log2g);
+    const bool vec = choose_io_shape(a).vec, pdl = (a->launch_flags & GRG_B200_LAUNCH_PDL) != 0;
+    GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, mx_encode_rows_kernel, static_cast<const double*>(a->input), a->ld_input, a->num_mutations, a->k, vec,
+                          static_cast<uint32_t*>(const_cast<void*>(la.x)), static_cast<uint16_t*>(const_cast<void*>(la.x_lo)), ld, log2g));
     GRG_LAUNCH_CHECK("mx_encode_rows_kernel(input)");
     if (a->use_miss) {
-        mx_encode_rows_kernel<<<grid, 256, 0, s>>>(static_cast<const double*>(a->miss), a->ld_miss, a->num_mutations, a->k,
-                                                   static_cast<uint32_t*>(const_cast<void*>(la.miss)),
-                                                   static_cast<uint16_t*>(const_cast<void*>(la.miss_lo)), ld, log2g);
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, mx_encode_rows_kernel, static_cast<const double*>(a->miss), a->ld_miss, a->num_mutations, a->k, vec,
+                              static_cast<uint32_t*>(const_cast<void*>(la.miss)), static_cast<uint16_t*>(const_cast<void*>(la.miss_lo)), ld, log2g));
         GRG_LAUNCH_CHECK("mx_encode_rows_kernel(miss)");
     }
     return GRG_B200_OK;

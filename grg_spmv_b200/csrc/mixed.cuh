@@ -69,15 +69,25 @@ __device__ __forceinline__ void mx_store(uint32_t* hi_row, uint16_t* lo_row, con
     *reinterpret_cast<uint2*>(lo_row) = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
 }
 
-// Columns [c, c + 4) of an FP64 row with columns >= k read as zero.
-__device__ __forceinline__ Quad f64_load_guarded(const double* row, int64_t c, int64_t k) {
+// Columns [c, c + 4) of an FP64 row, columns >= k read as zero and not written: two 16-byte accesses
+// where `vec` says that k, the stride and the base allow them.
+__device__ __forceinline__ Quad f64_load(const double* row, int64_t c, int64_t k, bool vec) {
     Quad q;
+    if (vec) {
+        const Pack<double, 2> lo = ld_ro<double, 2>(row + c), hi = ld_ro<double, 2>(row + c + 2);
+        return Quad{{lo.v[0], lo.v[1], hi.v[0], hi.v[1]}};
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) q.v[i] = c + i < k ? __ldg(row + c + i) : 0.0;
     return q;
 }
 
-__device__ __forceinline__ void f64_store_guarded(double* row, int64_t c, int64_t k, const Quad& q) {
+__device__ __forceinline__ void f64_store(double* row, int64_t c, int64_t k, bool vec, const Quad& q) {
+    if (vec) {
+        st_pack(row + c, Pack<double, 2>{{q.v[0], q.v[1]}});
+        st_pack(row + c + 2, Pack<double, 2>{{q.v[2], q.v[3]}});
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
         if (c + i < k) row[c + i] = q.v[i];
@@ -85,7 +95,7 @@ __device__ __forceinline__ void f64_store_guarded(double* row, int64_t c, int64_
 
 // Columns [c, c + 4) of a node's init value.
 __device__ __forceinline__ Quad mx_init(const LevelArgs& a, int init_mode, int64_t row, int64_t c) {
-    if (init_mode == GRG_B200_INIT_VECTOR) return f64_load_guarded(static_cast<const double*>(a.init_vector), c, a.k);
+    if (init_mode == GRG_B200_INIT_VECTOR) return f64_load(static_cast<const double*>(a.init_vector), c, a.k, false);
     if (init_mode == GRG_B200_INIT_XTX) {
         const double x = __ldg(static_cast<const double*>(a.xtx_node) + row);
         return Quad{{x, x, x, x}};
@@ -96,7 +106,7 @@ __device__ __forceinline__ Quad mx_init(const LevelArgs& a, int init_mode, int64
             report(a.err, kErrPerm);
             return zero_quad();
         }
-        return f64_load_guarded(static_cast<const double*>(a.init_matrix) + orig * a.ld_init, c, a.k);
+        return f64_load(static_cast<const double*>(a.init_matrix) + orig * a.ld_init, c, a.k, false);
     }
     return zero_quad();
 }
