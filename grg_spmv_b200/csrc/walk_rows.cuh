@@ -338,13 +338,14 @@ int launch_rows(const LevelArgs& la, int init_mode, int64_t num_entries, const i
     // Heavy rows: more warps a row while the rows alone leave the GPU idle.
     ws.heavy_warps = 1;
     while (ws.heavy_warps < nw && la.num_heavy * ws.heavy_warps * 2 <= kResidentWarps) ws.heavy_warps *= 2;
-    // Rows left to one CTA must not outlast their level: those of 16 rounds of fetches and more, and
-    // more than twice the level's own rounds per warp, go to clusters.  A 10,491-entry row at
+    // Rows left to one CTA must not outlast their level: those of 8 rounds of fetches and more, and
+    // more than twice the level's own rounds per warp, go to clusters (at 16: 80k nodes down k = 1 35.1
+    // us, at 8: 32.8; at 32: k = 4 47.1 against 36.9).  A 10,491-entry row at
     // k = 64 held one warp for 1477 us (the whole down traversal of 600k nodes: 2423 us, now 601).
     const int64_t level_rounds = num_entries / (4 * ws.groups) / kResidentWarps;
     for (int i = 0; i < GRG_B200_LONG_CLASSES && ws.hubs == 0; ++i) {
         const int64_t rounds = (int64_t{GRG_B200_LONG_ROW} << i) / (4 * ws.groups * ws.heavy_warps);
-        if (rounds >= 16 && rounds > 2 * level_rounds) ws.hubs = static_cast<int>(long_counts[i]);
+        if (rounds >= 8 && rounds > 2 * level_rounds) ws.hubs = static_cast<int>(long_counts[i]);
     }
     if (ws.hubs > 0)
         GRG_CUDA_TRY(launch_k(pdl, s, dim3(static_cast<unsigned>(ws.hubs * kHubCtas)), 32 * kHubWarps, level_hub_kernel<H>, la, ws));
