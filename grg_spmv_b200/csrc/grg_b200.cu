@@ -1551,55 +1551,32 @@ __device__ __forceinline__ Quad mx_state_row(const OutArgs& a, int64_t n, int64_
     return mx_load(static_cast<const uint32_t*>(a.state) + o, static_cast<const uint16_t*>(a.state_lo) + o);
 }
 
-// As gather_out_kernel: R rows per lane group, their extents and first indexes loaded before the
-// wait and their first state rows in flight together.
-template <bool BIAS_PER_ENTRY, int R>
+// One row per lane group, its extent and first index loaded before the wait.  Four rows, as
+// gather_out_kernel takes, lose here to the decoding's registers (1.5M nodes up k = 31: 525 -> 541 us).
+template <bool BIAS_PER_ENTRY>
 __global__ void __launch_bounds__(256) gather_out_mx_kernel(OutArgs a) {
-    const int per_block = 256 >> a.log2g;
-    const int lane = static_cast<int>(threadIdx.x) & ((1 << a.log2g) - 1);
-    const int64_t first = static_cast<int64_t>(blockIdx.x) * per_block * R + (threadIdx.x >> a.log2g);
-    int32_t e0[R], e1[R];
-    int64_t n0[R];
-#pragma unroll
-    for (int u = 0; u < R; ++u) {
-        const int64_t r = first + static_cast<int64_t>(u) * per_block;
-        e0[u] = r < a.rows ? __ldg(a.ptr + r) : 0;
-        e1[u] = r < a.rows ? __ldg(a.ptr + r + 1) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < R; ++u) n0[u] = e0[u] < e1[u] ? __ldg(a.idx + e0[u]) : 0;
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t r = t >> a.log2g;
+    if (r >= a.rows) return;
+    const int lane = static_cast<int>(t & ((1 << a.log2g) - 1));
+    const int32_t e0 = __ldg(a.ptr + r), e1 = __ldg(a.ptr + r + 1);
+    const int64_t n0 = e0 < e1 ? __ldg(a.idx + e0) : 0;
     pdl_wait();
     double* out = static_cast<double*>(a.out);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
-        Quad v[R];
-#pragma unroll
-        for (int u = 0; u < R; ++u) {
-            v[u] = zero_quad();
-            if (e0[u] < e1[u]) {
-                if (a.err && (n0[u] < 0 || n0[u] >= a.lim)) report(a.err, kErrSelector);
-                else v[u] = mx_state_row(a, n0[u], c);
+        Quad s = zero_quad();
+        for (int32_t e = e0; e < e1; ++e) {
+            const int64_t n = e == e0 ? n0 : __ldg(a.idx + e);
+            if (a.err && (n < 0 || n >= a.lim)) {
+                report(a.err, kErrSelector);
+                continue;
             }
+            Quad v = mx_state_row(a, n, c);
+            if constexpr (BIAS_PER_ENTRY) mx_apply_bias(a, n, c, v);
+            add_quad(s, v);
         }
-#pragma unroll
-        for (int u = 0; u < R; ++u) {
-            const int64_t r = first + static_cast<int64_t>(u) * per_block;
-            if (r < a.rows) {
-                Quad s = zero_quad();
-                for (int32_t e = e0[u]; e < e1[u]; ++e) {
-                    int64_t n = n0[u];
-                    if (e > e0[u]) n = __ldg(a.idx + e);
-                    if (a.err && (n < 0 || n >= a.lim)) {
-                        report(a.err, kErrSelector);
-                        continue;
-                    }
-                    if (e > e0[u]) v[u] = mx_state_row(a, n, c);
-                    if constexpr (BIAS_PER_ENTRY) mx_apply_bias(a, n, c, v[u]);
-                    add_quad(s, v[u]);
-                }
-                if constexpr (!BIAS_PER_ENTRY) mx_apply_bias(a, r, c, s);
-                f64_store(out + r * a.ld_out, c, a.k, a.vec, s);
-            }
-        }
+        if constexpr (!BIAS_PER_ENTRY) mx_apply_bias(a, r, c, s);
+        f64_store(out + r * a.ld_out, c, a.k, a.vec, s);
     }
 }
 
@@ -2280,13 +2257,6 @@ OutArgs out_args(const grg_b200_traverse_args* a, const IoShape& io) {
     return o;
 }
 
-template <bool BIAS_PER_ENTRY>
-cudaError_t launch_gather_out_mx(bool pdl, cudaStream_t s, const OutArgs& o) {
-    if ((o.rows << o.log2g) <= int64_t{148} * 2048)
-        return launch_k(pdl, s, grid_for(o.rows, o.log2g, 256), 256, gather_out_mx_kernel<BIAS_PER_ENTRY, 1>, o);
-    return launch_k(pdl, s, grid_for((o.rows + kOutRows - 1) / kOutRows, o.log2g, 256), 256, gather_out_mx_kernel<BIAS_PER_ENTRY, kOutRows>, o);
-}
-
 template <typename T, int V, bool BIAS_PER_ENTRY>
 cudaError_t launch_gather_out(bool pdl, cudaStream_t s, const OutArgs& o) {
     if ((o.rows << o.log2g) <= int64_t{148} * 2048)
@@ -2308,7 +2278,7 @@ int output_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
     o.idx = a->sel_mut_idx;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        GRG_CUDA_TRY(launch_gather_out_mx<false>(pdl, s, o));
+        GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, o));
         GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_mut)");
         if (a->use_miss) {
             OutArgs m = o;
@@ -2317,7 +2287,7 @@ int output_up_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
             m.out = a->miss;
             m.ld_out = a->ld_miss;
             m.bias_mode = GRG_B200_BIAS_NONE;
-            GRG_CUDA_TRY(launch_gather_out_mx<false>(pdl, s, m));
+            GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<false>, m));
             GRG_LAUNCH_CHECK("gather_out_mx_kernel(sel_miss)");
         }
         return (int)GRG_B200_OK;
@@ -2359,7 +2329,7 @@ int output_down_impl(const grg_b200_traverse_args* a, cudaStream_t s) {
     if (o.rows == 0) return GRG_B200_OK;
     const dim3 grid = grid_for(o.rows, o.log2g, 256);
     if (a->dtype == GRG_B200_MIXED) {
-        if (a->by_individual) GRG_CUDA_TRY(launch_gather_out_mx<true>(pdl, s, o));
+        if (a->by_individual) GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, gather_out_mx_kernel<true>, o));
         else GRG_CUDA_TRY(launch_k(pdl, s, grid, 256, copy_out_mx_kernel, o));
         GRG_LAUNCH_CHECK("output_down_mx");
         return (int)GRG_B200_OK;
