@@ -106,7 +106,7 @@ def parse_args():
     p.add_argument("--schedule", choices=["levels", "dataflow"], default=None,
                    help="one launch per level, or one persistent dataflow launch per traversal")
     p.add_argument("--precision", choices=["plain", "mixed"], default="plain",
-                   help="node state in FP64 (plain) or FP32 + 16-bit correction with FP64 sums (mixed)")
+                   help="node state in FP64 (plain) or FP32 + 16 more mantissa bits with FP64 sums (mixed)")
     p.add_argument("--row-order-up", choices=["natural", "locality"], default=None)
     p.add_argument("--row-order-down", choices=["natural", "locality"], default=None)
     p.add_argument("--apps", action="store_true",
@@ -244,7 +244,7 @@ CONFIG2_K8_TRAFFIC = {
     ("down", 1): {"kernel": "level_entry_pre_kernel", "dram_bytes": 525780224 + 21631744, "ncu_us": 110.72},
     ("down", 0): {"kernel": "level_lean_warp_kernel", "dram_bytes": 458001152 + 17115392, "ncu_us": 208.93},
 }
-CONFIG2_K8_VARIANT = 15  # the narrow variant those launches ran
+CONFIG2_K8_VARIANT = 15  # the narrow variant those launches ran (named by the plan; default plans run the row walk)
 TRAFFIC_SOURCE = "profiles/level_traffic_config2_k8.md (ncu -c 1 per launch on the config-2 graph, k = 8)"
 
 
@@ -687,7 +687,8 @@ def run_b200(args) -> None:
     traffic, traffic_launches = None, None
     captured = (args.workload == "config2" and k == 8 and args.precision == "plain" and pair.plan_down.schedule == "levels"
                 and not args.heavy_buckets and not args.no_short_rows and launch_ms
-                and narrow_used == {"up": CONFIG2_K8_VARIANT, "down": CONFIG2_K8_VARIANT})
+                and narrow_used == {"up": CONFIG2_K8_VARIANT, "down": CONFIG2_K8_VARIANT}
+                and not (pair.plan_up.library_walk() or pair.plan_down.library_walk()))
     if captured:
         traffic_launches = []
         for (direction, level), cap in CONFIG2_K8_TRAFFIC.items():
@@ -1095,7 +1096,7 @@ def run_precision(args, timed, device) -> dict:
     """The precision configuration: the config-2 graph in its diploid variant with coalescence
     counts, k = 32, up and down with init_xtx (the 2·coalescence-count node initialisation and
     its endpoint bias, in FP64), N(0,1) and integer allele-count (0, 1, 2) inputs.  The node
-    state in plain FP64 and in the mixed format (FP32 + 16-bit correction, FP64 sums); device
+    state in plain FP64 and in the mixed format (FP32 + 16 more mantissa bits, FP64 sums); device
     time per up+down pair and the max relative error of each against the CPU oracle (FP64, the
     reference's arithmetic) on the first 4 of the 32 columns, and of mixed against plain FP64 on
     all 32."""
