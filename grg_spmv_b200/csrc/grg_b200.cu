@@ -1016,6 +1016,7 @@ __global__ void __launch_bounds__(256) seed_up_mx_kernel(LevelArgs a, bool vec, 
             return;
         }
     }
+    pdl_wait();  // inputs, init values and the state it overwrites belong to earlier kernels
     const double* x = static_cast<const double*>(a.x);
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < a.k; c += static_cast<int64_t>(4) << a.log2g) {
         Quad v = mx_init(a, init_mode, row, c);

@@ -1,0 +1,68 @@
+"""Mixed storage on the paths that ordinary calls take: no bounds checks, recorded and captured calls.
+
+Integer-valued inputs are exact (sums stay below 2^40).  Real ones: each node is rounded to within
+2^-40 of itself, a path has at most 12 nodes here, and the FP64 sums add less than 1e-11 (2^16 terms),
+so a result is within 1e-10 of the largest magnitude sum."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+from grg_oracle import OracleGRG  # noqa: E402
+from grg_spmv_b200 import RuntimeRequirements  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def artifact(tmp_path_factory):
+    """Diploid, random ids, thousands of mutations on one node (rows of every kind of walk)."""
+    from grg_spmv_b200.synth import SynthSpec, write_synthetic_artifact
+
+    path = tmp_path_factory.mktemp("mixed_paths") / "mixed.grg_spmv"
+    write_synthetic_artifact(SynthSpec(num_samples=1200, num_levels=12, num_nodes=60_000, num_mutations=40_000, children=(2, 14),
+                                       miss_fraction=0.02, ploidy=2, with_coalescence=True, random_ids=True, seed=41), path)
+    return path
+
+
+def _runtime(path, k, stream=0, **kw):
+    from grg_spmv_b200.backends.b200 import B200Runtime, plan_b200_layout
+
+    req = RuntimeRequirements(max_k_up=k, max_k_down=k, need_down_miss_input=True, need_up_miss_output=True,
+                              need_init_vector=True, need_init_matrix=False, need_init_xtx=True)
+    layout = plan_b200_layout(artifacts=[str(path)], dtype=np.float64, requirements=req, vram_budget_bytes=0, ring_buffer_size=0,
+                              device=0, stream=stream, precision="mixed")
+    return B200Runtime(layout, check_bounds=False, **kw)
+
+
+@pytest.mark.parametrize("k", [1, 8])
+@pytest.mark.parametrize("init", ["none", "vector"])
+def test_mixed_up_captured_after_the_kernel_that_writes_its_input(artifact, init, k):
+    """The caller's graph: a kernel writes the input, the traversal reads it, another kernel
+    overwrites it (and so on, twice), all in one capture."""
+    oracle = OracleGRG(artifact)
+    rng = np.random.default_rng(17)
+    stream = torch.cuda.Stream(device=0)
+    with _runtime(artifact, k, stream) as runtime:
+        (grg,) = runtime.grgs
+        xs = [rng.integers(-4, 5, size=(k, grg.num_samples)).astype(np.float64) for _ in range(2)]
+        v = rng.integers(-4, 5, size=k).astype(np.float64)
+        op = grg.prepare_matmul_cuda(direction="up", k=k, init_mode=init)
+        halves = [torch.from_numpy(x / 2).to("cuda:0") for x in xs]
+        outs = [torch.empty((k, grg.num_mutations), device="cuda:0", dtype=torch.float64) for _ in xs]
+        if init == "vector":
+            op.init_vector.copy_(torch.from_numpy(v))
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for half, out in zip(halves, outs):
+                torch.add(half, half, out=op.input)
+                op()
+                out.copy_(op.output)
+        for _ in range(3):
+            graph.replay()
+        torch.cuda.synchronize()
+        for x, out in zip(xs, outs):
+            np.testing.assert_array_equal(out.cpu().numpy(), oracle.matmul(x, "up", init=v if init == "vector" else None))
