@@ -988,7 +988,8 @@ __global__ void __launch_bounds__(kNarrowThreads, MB) level_run_kernel(const __g
 // Mixed storage (dtype GRG_B200_MIXED, mixed.cuh): inputs in and out.  A buffer of R rows and ld
 // columns (ld % 4 == 0) is two planes: uint32 hi[R * ld] followed by uint16 lo[R * ld].
 // ---------------------------------------------------------------------------------------
-// Encoded copy of an FP64 matrix: dst[r, c] = src[r, c] for c < k, 0 for k <= c < ld.
+// Encoded copy of an FP64 matrix: dst[r, c] = src[r, c] for c < k, 0 for k <= c < ld (ld may be any
+// multiple of 4 from k on; `vec` says that k is one too, so a quad is inside a source row or past it).
 __global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, int64_t ld_src, int64_t rows, int64_t k, bool vec,
                                                              uint32_t* dst_hi, uint16_t* dst_lo, int64_t ld, int32_t log2g) {
     pdl_trigger();
@@ -998,7 +999,7 @@ __global__ void __launch_bounds__(256) mx_encode_rows_kernel(const double* src, 
     if (r >= rows) return;
     const int lane = static_cast<int>(t & ((1 << log2g) - 1));
     for (int64_t c = static_cast<int64_t>(lane) * 4; c < ld; c += static_cast<int64_t>(4) << log2g)
-        mx_store(dst_hi + r * ld + c, dst_lo + r * ld + c, f64_load(src + r * ld_src, c, k, vec));
+        mx_store(dst_hi + r * ld + c, dst_lo + r * ld + c, f64_load(src + r * ld_src, c, k, vec && c < k));
 }
 
 // Up seeding of level 0 in mixed storage: state[r] = init(r) (+ input row for samples).

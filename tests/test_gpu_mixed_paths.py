@@ -66,3 +66,40 @@ def test_mixed_up_captured_after_the_kernel_that_writes_its_input(artifact, init
         torch.cuda.synchronize()
         for x, out in zip(xs, outs):
             np.testing.assert_array_equal(out.cpu().numpy(), oracle.matmul(x, "up", init=v if init == "vector" else None))
+
+
+def test_mixed_down_with_a_state_wider_than_k(artifact):
+    """ld_state > k through the C interface: the encoded copies hold zeros from column k on, and no
+    column past a source row is read (what follows the inputs is NaN here)."""
+    import ctypes
+
+    from grg_spmv_b200.backends.b200 import _native as nat
+
+    k, ld = 8, 16
+    oracle = OracleGRG(artifact)
+    rng = np.random.default_rng(29)
+    with _runtime(artifact, k) as runtime:
+        (grg,) = runtime.grgs
+        M, N = grg.num_mutations, grg.num_nodes
+        args = grg.prepare_matmul_cuda(direction="down", k=k, use_miss=True)._args
+        x, miss = (rng.integers(-4, 5, size=(M, k)).astype(np.float64) for _ in range(2))
+        buffers = []
+        for values in (x, miss):
+            buf = torch.full((M + 2, k), float("nan"), device="cuda:0", dtype=torch.float64)
+            buf[:M] = torch.from_numpy(values)
+            buffers.append(buf)
+        state = torch.zeros(nat.mix_bytes(N, ld), device="cuda:0", dtype=torch.uint8)
+        scratch = torch.full((2 * nat.mix_bytes(M, ld),), 0x55, device="cuda:0", dtype=torch.uint8)
+        out = torch.empty((grg.num_samples, k), device="cuda:0", dtype=torch.float64)
+        args.input, args.miss, args.output = (t.data_ptr() for t in (*buffers, out))
+        args.ld_input = args.ld_miss = args.ld_output = k
+        args.state, args.ld_state = state.data_ptr(), ld
+        args.mix_scratch, args.mix_scratch_bytes = scratch.data_ptr(), scratch.numel()
+        torch.cuda.synchronize()
+        nat.check(runtime._lib, runtime._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(runtime.stream_ptr)), "traverse")
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy().T, oracle.matmul(x.T.copy(), "down", miss=miss.T.copy()))
+        for part in scratch.cpu().numpy().reshape(2, -1):
+            hi = part[: M * ld * 4].view(np.uint32).reshape(M, ld)
+            lo = part[nat.mix_plane(M * ld * 4):][: M * ld * 2].view(np.uint16).reshape(M, ld)
+            assert not hi[:, k:].any() and not lo[:, k:].any()
