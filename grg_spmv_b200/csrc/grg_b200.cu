@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kNarrowThreads, MIN_BLOCKS) level_narrow_kerne
             for (int u = 0; u < U; ++u) {
                 const T* src = (e + u < e1) ? entry_row<T>(a, code[u]) : nullptr;
                 valid[u] = src != nullptr;
-                val[u] = valid[u] ? ld_ro<T, V>(src + c) : zero_pack<T, V>();
+                val[u] = valid[u] ? ld_row<T, V>(src + c) : zero_pack<T, V>();
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
@@ -350,7 +350,7 @@ __device__ __forceinline__ void split_rows(const LevelArgs& a, int64_t block) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const T* src = entry_row<T>(a, code[u]);
-                    val[u] = src ? ld_ro<T, V>(src + c) : zero_pack<T, V>();
+                    val[u] = src ? ld_row<T, V>(src + c) : zero_pack<T, V>();
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) add_into(part, val[u]);
@@ -516,7 +516,7 @@ __device__ __forceinline__ void lean_rows(const LevelArgs& a, int64_t block) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const T* p = lean_source<T, UPONLY>(a, code[u], ok[u]);
-                val[u] = ok[u] ? ld_ro<T, V>(p + c) : zero_pack<T, V>();
+                val[u] = ok[u] ? ld_row<T, V>(p + c) : zero_pack<T, V>();
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -573,7 +573,7 @@ __device__ __forceinline__ void lean_heavy_rows(const LevelArgs& a, int64_t bloc
                 for (int u = 0; u < 4; ++u) {
                     bool ok;
                     const T* p = lean_source<T, UPONLY>(a, code[u], ok);
-                    val[u] = ok ? ld_ro<T, V>(p + c) : zero_pack<T, V>();
+                    val[u] = ok ? ld_row<T, V>(p + c) : zero_pack<T, V>();
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) add_into(part, val[u]);
@@ -877,7 +877,7 @@ __device__ __forceinline__ void persist_rows(const LevelArgs& a, int32_t block, 
                 for (int u = 0; u < 4; ++u) {
                     const T* src = entry_row<T>(a, code[u]);
                     valid[u] = src != nullptr;
-                    val[u] = valid[u] ? ld_ro<T, V>(src + c) : zero_pack<T, V>();
+                    val[u] = valid[u] ? ld_row<T, V>(src + c) : zero_pack<T, V>();
                 }
                 if (pending) {  // after this round's fetches are issued: waits only on n0
                     nfirst = (n0 >> 2) < (n1 >> 2) ? __ldg(codes4 + (n0 >> 2)) : null4;
@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(kWideThreads) level_wide_kernel(LevelArgs a) {
                         for (int u = 0; u < UW; ++u) {
                             const int jj = j + u * groups;
                             const T* src = jj < n ? entry_row<T>(a, codes[jj]) : nullptr;
-                            val[u] = src ? ld_ro<T, V>(src + c) : zero_pack<T, V>();
+                            val[u] = src ? ld_row<T, V>(src + c) : zero_pack<T, V>();
                         }
 #pragma unroll
                         for (int u = 0; u < UW; ++u) add_into(part, val[u]);
@@ -1099,7 +1099,7 @@ __global__ void __launch_bounds__(kWideThreads) level_wide_kernel(LevelArgs a) {
                 if (e < e1) {
                     code = __ldg(a.entries + e);
                     const T* src = entry_row<T>(a, code);
-                    if (src && active) val = ld_ro<T, V>(src + c);
+                    if (src && active) val = ld_row<T, V>(src + c);
                 }
                 red[threadIdx.x] = val;
                 if (lane == 0) codes[grp] = code;
@@ -1215,7 +1215,7 @@ __device__ __forceinline__ Pack<T, V> df_fetch(const DfArgs& p, uint32_t code, i
         return v;
     }
     const T* row = entry_row<T>(p.a, code);
-    return row ? ld_ro<T, V>(row + c) : zero_pack<T, V>();
+    return row ? ld_row<T, V>(row + c) : zero_pack<T, V>();
 }
 
 template <typename T, int V, int INIT>
@@ -1340,10 +1340,10 @@ __global__ void __launch_bounds__(256) sentinel_fill_kernel(T* state, int64_t n)
 // the bases allow it, else value by value up to k.  State rows hold whole vectors either way.
 template <typename T, int V>
 __device__ __forceinline__ Pack<T, V> ld_io(const T* row, int64_t c, int64_t k, bool vec) {
-    if (vec) return ld_ro<T, V>(row + c);
+    if (vec) return ld_row<T, V>(row + c);
     Pack<T, V> r;
 #pragma unroll
-    for (int i = 0; i < V; ++i) r.v[i] = c + i < k ? __ldg(row + c + i) : T(0);
+    for (int i = 0; i < V; ++i) r.v[i] = c + i < k ? ld_row<T, 1>(row + c + i).v[0] : T(0);
     return r;
 }
 
@@ -1466,7 +1466,7 @@ __global__ void __launch_bounds__(256) gather_out_kernel(OutArgs a) {
             v[u] = zero_pack<T, V>();
             if (e0[u] < e1[u]) {
                 if (a.err && (n0[u] < 0 || n0[u] >= a.lim)) report(a.err, kErrSelector);
-                else v[u] = ld_ro<T, V>(state + n0[u] * a.ld_state + c);
+                else v[u] = ld_row<T, V>(state + n0[u] * a.ld_state + c);
             }
         }
 #pragma unroll
@@ -1482,7 +1482,7 @@ __global__ void __launch_bounds__(256) gather_out_kernel(OutArgs a) {
                             report(a.err, kErrSelector);
                             continue;
                         }
-                        v[u] = ld_ro<T, V>(state + n * a.ld_state + c);
+                        v[u] = ld_row<T, V>(state + n * a.ld_state + c);
                     } else if (a.err && (n < 0 || n >= a.lim)) {
                         continue;
                     }
@@ -1508,7 +1508,7 @@ __global__ void __launch_bounds__(256) copy_out_kernel(OutArgs a) {
     T* out = static_cast<T*>(a.out);
     const int64_t step = static_cast<int64_t>(V) << a.log2g;
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step) {
-        Pack<T, V> v = ld_ro<T, V>(state + r * a.ld_state + c);
+        Pack<T, V> v = ld_row<T, V>(state + r * a.ld_state + c);
         apply_bias<T, V>(a, r, c, v);
         st_io(out + r * a.ld_out, c, a.k, a.vec, v);
     }
@@ -1531,7 +1531,7 @@ __global__ void __launch_bounds__(256) emit_all_kernel(OutArgs a) {
     T* out = static_cast<T*>(a.out);
     const int64_t step = static_cast<int64_t>(V) << a.log2g;
     for (int64_t c = static_cast<int64_t>(lane) * V; c < a.k; c += step)
-        st_io(out + j * a.ld_out, c, a.k, a.vec, ld_ro<T, V>(state + n * a.ld_state + c));
+        st_io(out + j * a.ld_out, c, a.k, a.vec, ld_row<T, V>(state + n * a.ld_state + c));
 }
 
 // Output kernels for mixed storage: decode to FP64, 4 columns per lane, columns >= k skipped.
@@ -2502,7 +2502,7 @@ __global__ void __launch_bounds__(kRowopThreads, 3) rowop_kernel(grg_b200_rowop_
         const bool active = j < a.k;
         Pack<double, V> part = zero_pack<double, V>();
         if (active) {
-            const Pack<double, V> cs = a.col_sub ? ld_ro<double, V>(a.col_sub + j) : zero_pack<double, V>();
+            const Pack<double, V> cs = a.col_sub ? ld_row<double, V>(a.col_sub + j) : zero_pack<double, V>();
             for (int64_t r = r0 + ty; r < r1; r += static_cast<int64_t>(kRowopUnroll) * ny) {
                 // src may be dst and miss_in may be miss_out: every element is read before it is
                 // written, by this thread, so plain loads

@@ -33,7 +33,7 @@ __device__ __forceinline__ Pack<T, CW> fetch(const LevelArgs& a, uint32_t code, 
         if (ok && ((code >> GRG_B200_SRC_SHIFT) & GRG_B200_SRC_MASK) != GRG_B200_SRC_STATE) {
             Pack<T, CW> r;
 #pragma unroll
-            for (int i = 0; i < CW; ++i) r.v[i] = c + i < a.k ? __ldg(p + c + i) : T(0);
+            for (int i = 0; i < CW; ++i) r.v[i] = c + i < a.k ? ld_row<T, 1>(p + c + i).v[0] : T(0);
             return r;
         }
     }

@@ -22,8 +22,8 @@ struct MxRaw {
 };
 
 __device__ __forceinline__ MxRaw mx_ld(const uint32_t* hi, const uint16_t* lo) {
-    const uint4 h = __ldg(reinterpret_cast<const uint4*>(hi));
-    const uint2 l = __ldg(reinterpret_cast<const uint2*>(lo));
+    const uint4 h = ld_words4(hi);
+    const uint2 l = ld_words2(lo);
     return MxRaw{{h.x, h.y, h.z, h.w}, {l.x, l.y}};
 }
 

@@ -56,8 +56,8 @@ __device__ __forceinline__ void add_quad(Quad& a, const Quad& b) {
 
 // Four columns as a 16-byte hi and an 8-byte lo load or store.
 __device__ __forceinline__ Quad mx_load(const uint32_t* hi_row, const uint16_t* lo_row) {
-    const uint4 h = __ldg(reinterpret_cast<const uint4*>(hi_row));
-    const uint2 l = __ldg(reinterpret_cast<const uint2*>(lo_row));
+    const uint4 h = ld_words4(hi_row);
+    const uint2 l = ld_words2(lo_row);
     return Quad{{mx_decode(h.x, l.x & 0xffffu), mx_decode(h.y, l.x >> 16), mx_decode(h.z, l.y & 0xffffu), mx_decode(h.w, l.y >> 16)}};
 }
 
@@ -74,11 +74,11 @@ __device__ __forceinline__ void mx_store(uint32_t* hi_row, uint16_t* lo_row, con
 __device__ __forceinline__ Quad f64_load(const double* row, int64_t c, int64_t k, bool vec) {
     Quad q;
     if (vec) {
-        const Pack<double, 2> lo = ld_ro<double, 2>(row + c), hi = ld_ro<double, 2>(row + c + 2);
+        const Pack<double, 2> lo = ld_row<double, 2>(row + c), hi = ld_row<double, 2>(row + c + 2);
         return Quad{{lo.v[0], lo.v[1], hi.v[0], hi.v[1]}};
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) q.v[i] = c + i < k ? __ldg(row + c + i) : 0.0;
+    for (int i = 0; i < 4; ++i) q.v[i] = c + i < k ? ld_row<double, 1>(row + c + i).v[0] : 0.0;
     return q;
 }
 

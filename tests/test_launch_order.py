@@ -54,3 +54,15 @@ def test_kernels_launched_early_wait_for_the_previous_grid():
 
     assert sorted(k for k in kernels if not waits(k)) == []
     assert sorted(k for k, body in bodies.items() if "pdl_trigger()" in body and k != "pdl_trigger" and not waits(k)) == []
+
+
+def test_read_only_loads_name_static_arrays():
+    """A read-only load may be served by a line from before the previous grid's writes, and may be
+    moved ahead of the wait: only lists, selectors, permutations and per-row constants take it."""
+    text = _source()
+    assert "ld.global.nc" not in text
+    static = r"(?:[aL]\.)?(?:row_ptr|row_ids|entries|heavy_rows|codes4?|ptr|idx|node_perm|s2i|xtx_node|bias|(?:pre|sub|post|miss|miss_out)_scale|sum_weight)"
+    loads = [text[m.end():_closing(text, m.end() - 1, "()") - 1] for m in re.finditer(r"__ldg\(", text)]
+    assert len(loads) > 20
+    unknown = [arg for arg in loads if not re.match(static + r"\b", re.sub(r"^(?:static_cast|reinterpret_cast)<[^>]*>+\(", "", arg))]
+    assert unknown == []
