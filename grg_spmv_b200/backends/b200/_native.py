@@ -32,6 +32,7 @@ F64, F32, MIXED = 0, 1, 2
 MAX_SLOT_BUCKETS = 8
 LAUNCH_PDL = 1
 LAUNCH_WALK = 2
+STATE_PADDING = 4
 LONG_ROW = 512
 LONG_CLASSES = 8
 QUAD_CLASSES = 8

@@ -508,6 +508,7 @@ class B200Runtime:
         else:  # whole vectors a row, where the state was planned with room for them
             padded = state_ld(k, self.layout.dtype.itemsize)
             a.ld_state = padded if state.numel() >= st.num_nodes * padded else k
+            a.launch_flags = nat.STATE_PADDING
         if mixed and mix_scratch is not None:
             a.mix_scratch = _ptr(mix_scratch)
             a.mix_scratch_bytes = int(mix_scratch.numel())
@@ -550,7 +551,7 @@ class B200Runtime:
         a.narrow_split = int(plan.narrow_split)
         a.persist_ctas = int(plan.persist_ctas)
         a.fuse_entries = int(plan.fuse_entries)
-        a.launch_flags = nat.LAUNCH_PDL if plan.resolve_pdl(k) else 0
+        a.launch_flags |= nat.LAUNCH_PDL if plan.resolve_pdl(k) else 0
         if plan.library_walk() and direction not in self._variant:
             a.launch_flags |= nat.LAUNCH_WALK | (nat.LAUNCH_PDL if plan.pdl is None else 0)
         a.schedule = nat.SCHEDULE_DATAFLOW if plan.schedule == "dataflow" else nat.SCHEDULE_LEVELS

@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(256) sentinel_fill_kernel(T* state, int64_t n)
 }
 
 // Columns [c, c + V) of an input or output row: one vector where `vec` says that k, the strides and
-// the bases allow it, else value by value up to k.  State rows hold whole vectors either way.
+// the bases allow it, else value by value up to k.  The call's state columns hold whole vectors either way.
 template <typename T, int V>
 __device__ __forceinline__ Pack<T, V> ld_io(const T* row, int64_t c, int64_t k, bool vec) {
     if (vec) return ld_row<T, V>(row + c);
@@ -1648,7 +1648,10 @@ Shape choose_shape(const grg_b200_traverse_args* a) {
     return {vec, log2g};
 }
 
-// Shape of the seed and output kernels: the widest vector that the state rows hold whole; `vec`
+// Columns of a state row that the call may touch.
+int64_t state_cols(const grg_b200_traverse_args* a) { return (a->launch_flags & GRG_B200_STATE_PADDING) ? a->ld_state : a->k; }
+
+// Shape of the seed and output kernels: the widest vector that the call's state columns hold whole; `vec`
 // says whether the input, output and init rows take it too.
 struct IoShape {
     Shape shape;
@@ -1665,7 +1668,9 @@ IoShape choose_io_shape(const grg_b200_traverse_args* a) {
     }
     const int esize = a->dtype == GRG_B200_F64 ? 8 : 4;
     int vec = 16 / esize;
-    while (vec > 1 && (a->ld_state % vec != 0 || !aligned(a->state, vec * esize) || a->k <= vec / 2)) vec >>= 1;
+    while (vec > 1 && (a->ld_state % vec != 0 || !aligned(a->state, vec * esize) || a->k <= vec / 2 ||
+                       (a->k + vec - 1) / vec * vec > state_cols(a)))
+        vec >>= 1;
     const int64_t lds[] = {a->ld_input, a->ld_output, a->use_miss ? a->ld_miss : 0, a->ld_init};
     const void* ptrs[] = {a->input, a->output, a->use_miss ? a->miss : nullptr, a->init_vector, a->init_matrix};
     bool whole = a->k % vec == 0;
@@ -1726,6 +1731,7 @@ LevelArgs level_args(const grg_b200_traverse_args* a, const Shape& sh) {
     la.use_miss = a->direction == GRG_B200_DOWN && a->use_miss;
     la.state = a->state;
     la.ld_state = a->ld_state;
+    la.state_cols = state_cols(a);
     la.x = a->input;
     la.ld_x = a->ld_input;
     la.miss = a->miss;
@@ -2970,6 +2976,7 @@ int grg_b200_traverse_static(const grg_b200_traverse_args* a, void* stream_handl
     while (padded < a->k && padded < chunk) padded <<= 1;
     if (a->k > chunk) padded = (a->k + chunk - 1) / chunk * chunk;
     local.ld_state = a->num_nodes <= (int64_t)GRG_B200_STATIC_STATE_BYTES / esize / padded ? padded : a->k;
+    local.launch_flags |= GRG_B200_STATE_PADDING;
     local.ring = nullptr;
     local.slot_buffers = nullptr;
     local.slot_bytes = nullptr;

@@ -176,6 +176,7 @@ struct LevelArgs {
     int32_t use_miss;
     void* state;
     int64_t ld_state;
+    int64_t state_cols;  // columns of a state row that belong to the call: k, or ld_state (GRG_B200_STATE_PADDING)
     const void* x;
     int64_t ld_x;
     const void* miss;

@@ -96,9 +96,11 @@ bool walk_serves(const LevelArgs& la, int init_mode, bool exact) {
 template <typename T>
 int launch_walk(const LevelArgs& la, int64_t num_entries, const int64_t* long_counts, bool pdl, cudaStream_t s) {
     constexpr int C = Chunk32<T>::C;
-    // the widest chunk that the state rows hold whole (their padding columns are scratch) and align
+    // the widest chunk that the call's state columns hold whole and that its rows align
     int cw = C;
-    while (cw > 1 && (la.ld_state % cw != 0 || !aligned(la.state, cw * static_cast<int>(sizeof(T))) || (cw > 1 && la.k <= cw / 2))) cw >>= 1;
+    while (cw > 1 && (la.ld_state % cw != 0 || !aligned(la.state, cw * static_cast<int>(sizeof(T))) || la.k <= cw / 2 ||
+                      (la.k + cw - 1) / cw * cw > la.state_cols))
+        cw >>= 1;
     const int64_t cols = (la.k + cw - 1) / cw * cw;  // columns that whole chunks touch
     const bool xv = cols == la.k && la.ld_x % cw == 0 && aligned(la.x, cw * static_cast<int>(sizeof(T))) &&
                     (!la.use_miss || (la.ld_miss % cw == 0 && aligned(la.miss, cw * static_cast<int>(sizeof(T)))));

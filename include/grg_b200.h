@@ -33,7 +33,8 @@
  *   grg_b200_last_error    - error reporting (the Python side raises RuntimeError with it).
  *
  * Data layout (all ids are positions in the artifact's stable height order):
- *   state   [num_nodes, ld_state]     node values, row-major
+ *   state   [num_nodes, ld_state]     node values, row-major; a call touches columns [0, k) (mixed:
+ *                                     k rounded up to 4), or all with GRG_B200_STATE_PADDING
  *   input   [rows, ld_input]          up: samples (or individuals), down: mutations
  *   output  [rows, ld_output]         up: mutations, down: samples (or individuals),
  *                                     emit_all_nodes: all nodes in ORIGINAL node order
@@ -264,7 +265,7 @@ typedef struct grg_b200_traverse_args {
     int32_t schedule;                   /* grg_b200_schedule */
     void* dataflow_sync;                /* GRG_B200_SCHEDULE_DATAFLOW and fused level runs: device int32[4], 16-byte aligned;
                                            [2] holds GRG_B200_DEVICE_WAIT_TIMEOUT after a failed wait */
-    int32_t launch_flags;               /* GRG_B200_LAUNCH_* bits */
+    int32_t launch_flags;               /* GRG_B200_LAUNCH_* and GRG_B200_STATE_PADDING bits */
     int32_t persist_ctas;               /* narrow_variant 9/10: CTAs of a level launch's persistent
                                            narrow part (each loops over row groups); 0 = what the
                                            GPU holds at once (SMs x CTAs per SM) */
@@ -287,6 +288,11 @@ typedef struct grg_b200_traverse_args {
  * (default mode, FP64/FP32, padded lists, no error word, no init inside the traversal; other
  * launches use narrow_variant and heavy_variant). */
 #define GRG_B200_LAUNCH_WALK 2
+
+/* Columns [k, ld_state) of the FP64/FP32 state rows belong to the call: kernels may read and write
+ * them, so rows of any k move in whole vectors where ld_state allows.  Without it a call touches
+ * columns [0, k) only, and several calls may keep their states in column slices of one buffer. */
+#define GRG_B200_STATE_PADDING 4
 
 /*
  * GRG_B200_SCHEDULE_LEVELS: one launch per level (each level waits for the previous one).
