@@ -195,6 +195,7 @@ class B200Runtime:
         self._grgs = ()
         self._variant = {}
         self._heavy_variant = {}
+        self._row_walk = {}
         self._entered = False
         self._active_call = False
 
@@ -256,7 +257,7 @@ class B200Runtime:
             for direction in (Direction.UP, Direction.DOWN):
                 plan = lay.pair.plan_for(direction)
                 if plan is not None and plan.autotune and lay.precision == "plain":
-                    self._variant[direction], self._heavy_variant[direction] = self._tune_direction(direction)
+                    self._variant[direction], self._heavy_variant[direction], self._row_walk[direction] = self._tune_direction(direction)
             self._entered = True
             return self
         except Exception:
@@ -390,12 +391,14 @@ class B200Runtime:
     # -- autotuning ------------------------------------------------------------------------------
     TUNE_VARIANTS = (5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 0, 1, 4)
 
-    def _tune_direction(self, direction: Direction) -> tuple[int, int]:
+    def _tune_direction(self, direction: Direction) -> tuple[int, int, bool]:
         """Fastest (narrow variant, heavy variant) for ``direction`` on the first artifact at
         the declared max k (the counterpart of ``TritonRuntime._tune_direction``,
-        ``pygrgl_spmv/backends/triton/backend.py:1062-1079``): narrow variants first, then the
-        two heavy-row kernels with the chosen narrow variant.  Each candidate runs once to warm
-        up and is then timed over three traversals with CUDA events."""
+        ``pygrgl_spmv/backends/triton/backend.py:1062-1079``), and whether the library's row walk
+        is at least as fast: narrow variants first, then the heavy-row kernels with the chosen
+        narrow variant, then the walk where it serves such calls.  Each candidate runs once to
+        warm up and is then timed over three traversals with CUDA events.  Calls that the walk
+        does not serve run the variants."""
         import torch
 
         from grg_spmv_b200.grg import CudaMatmulSpec
@@ -410,6 +413,8 @@ class B200Runtime:
                               apply_endpoint_bias=False)
         args = self._traverse_args(art, spec, self._io0[:cols_in, :k], self._io0[:cols_out, :k], None, None, None)
         plan = self.layout.pair.plan_for(direction)
+        walk_flags = args.launch_flags if args.launch_flags & nat.LAUNCH_WALK and not self._check_bounds else 0
+        args.launch_flags = self._launch_flags(plan, k, walk=False)
 
         def timed() -> float:
             self._launch(args)
@@ -433,7 +438,12 @@ class B200Runtime:
             for heavy in (0, 1, 2):
                 args.heavy_variant = heavy
                 heavy_ms[heavy] = timed()
-        return int(args.narrow_variant), int(min(heavy_ms, key=heavy_ms.get))
+            heavy = min(heavy_ms, key=heavy_ms.get)
+            row_walk = False
+            if walk_flags:
+                args.launch_flags = walk_flags
+                row_walk = timed() <= heavy_ms[heavy]
+        return int(args.narrow_variant), int(heavy), row_walk
 
     # -- calls ----------------------------------------------------------------------------------
     def _torch_caller_stream(self):
@@ -508,7 +518,6 @@ class B200Runtime:
         else:  # whole vectors a row, where the state was planned with room for them
             padded = state_ld(k, self.layout.dtype.itemsize)
             a.ld_state = padded if state.numel() >= st.num_nodes * padded else k
-            a.launch_flags = nat.STATE_PADDING
         if mixed and mix_scratch is not None:
             a.mix_scratch = _ptr(mix_scratch)
             a.mix_scratch_bytes = int(mix_scratch.numel())
@@ -551,12 +560,16 @@ class B200Runtime:
         a.narrow_split = int(plan.narrow_split)
         a.persist_ctas = int(plan.persist_ctas)
         a.fuse_entries = int(plan.fuse_entries)
-        a.launch_flags |= nat.LAUNCH_PDL if plan.resolve_pdl(k) else 0
-        if plan.library_walk() and direction not in self._variant:
-            a.launch_flags |= nat.LAUNCH_WALK | (nat.LAUNCH_PDL if plan.pdl is None else 0)
+        a.launch_flags = self._launch_flags(plan, k, walk=plan.library_walk() and self._row_walk.get(direction, True))
         a.schedule = nat.SCHEDULE_DATAFLOW if plan.schedule == "dataflow" else nat.SCHEDULE_LEVELS
         a.dataflow_sync = _ptr(self._df_sync if df_sync is None else df_sync)
         return a
+
+    def _launch_flags(self, plan, k: int, walk: bool) -> int:
+        flags = nat.STATE_PADDING  # the runtime's node states belong to one call at a time
+        if plan.resolve_pdl(k) or (walk and plan.pdl is None):
+            flags |= nat.LAUNCH_PDL
+        return flags | (nat.LAUNCH_WALK if walk else 0)
 
     def _capturing(self) -> bool:
         import torch
