@@ -81,8 +81,10 @@ class B200Plan:
     ``long_first``: with ``balance``, the longest length bucket is processed first.
     ``pdl``: launch the level, seed and output kernels with programmatic dependent launch
     (each overlaps the end of the previous one; ignored when levels are streamed).  None turns
-    it on for k >= 8, and for every k where the library chooses the row walk (measured on B200,
-    1.5M nodes, k = 1: up 178 -> 160 us, down 197 -> 153 us).
+    it on for k >= 8, and for every k where the library's row walk serves the call (measured on
+    B200, 1.5M nodes, k = 1: up 178 -> 160 us, down 197 -> 153 us).  The other kernels go without
+    below k = 8, where CTAs of the next level that are resident early crowd the short levels of a
+    large graph (1.5M nodes, up with a matrix init: k = 1 241 us without, 284 with; k = 2 291 and 360).
     ``slots``: with ``balance`` and ``pad_lists``, pad each narrow row to its bucket's width
     (1, 2, 4, 8 quads of 4 entries) so kernels locate its list from its position instead of
     loading ``row_ptr`` (one dependent load fewer per row, up to twice the list bytes).

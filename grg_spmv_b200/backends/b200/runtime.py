@@ -413,7 +413,7 @@ class B200Runtime:
                               apply_endpoint_bias=False)
         args = self._traverse_args(art, spec, self._io0[:cols_in, :k], self._io0[:cols_out, :k], None, None, None)
         plan = self.layout.pair.plan_for(direction)
-        walk_flags = args.launch_flags if args.launch_flags & nat.LAUNCH_WALK and not self._check_bounds else 0
+        walk_flags = args.launch_flags if args.launch_flags & nat.LAUNCH_WALK else 0
         args.launch_flags = self._launch_flags(plan, k, walk=False)
 
         def timed() -> float:
@@ -560,12 +560,15 @@ class B200Runtime:
         a.narrow_split = int(plan.narrow_split)
         a.persist_ctas = int(plan.persist_ctas)
         a.fuse_entries = int(plan.fuse_entries)
-        a.launch_flags = self._launch_flags(plan, k, walk=plan.library_walk() and self._row_walk.get(direction, True))
+        walk = plan.library_walk() and self._row_walk.get(direction, True)
+        served = mixed or (backend_init == InitMode.NONE and not self._check_bounds)
+        a.launch_flags = self._launch_flags(plan, k, walk=walk and served)
         a.schedule = nat.SCHEDULE_DATAFLOW if plan.schedule == "dataflow" else nat.SCHEDULE_LEVELS
         a.dataflow_sync = _ptr(self._df_sync if df_sync is None else df_sync)
         return a
 
     def _launch_flags(self, plan, k: int, walk: bool) -> int:
+        """``walk``: the library's row walk serves the call (mixed storage: every call)."""
         flags = nat.STATE_PADDING  # the runtime's node states belong to one call at a time
         if plan.resolve_pdl(k) or (walk and plan.pdl is None):
             flags |= nat.LAUNCH_PDL

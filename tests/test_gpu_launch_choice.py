@@ -67,3 +67,17 @@ def test_autotune_times_what_later_calls_run(artifact, checked):
             assert plain[1] == (not checked and runtime._row_walk[direction])
             for call in (plain, with_init):
                 assert call[2:] == (runtime._variant[direction], runtime._heavy_variant[direction])
+
+
+@pytest.mark.parametrize("precision,checked", [("plain", False), ("plain", True), ("mixed", False), ("mixed", True)])
+def test_early_launches_below_8_columns_where_the_row_walk_serves(artifact, precision, checked):
+    """Calls below k = 8 start levels early with the row walk only; from 8 on, and as a plan says, with any kernel."""
+    for pdl in (None, True, False):
+        pair = B200PlanPair(plan_up=B200Plan(pdl=pdl), plan_down=B200Plan(pdl=pdl))
+        with B200Runtime(_layout(artifact, 8, pair=pair, precision=precision), check_bounds=checked) as runtime:
+            (grg,) = runtime.grgs
+            for k in (1, 2, 7, 8):
+                for init, emit in (("none", False), ("none", True), ("matrix", False), ("vector", True)):
+                    op = grg.prepare_matmul_cuda(direction="up", k=k, init_mode=init, emit_all_nodes=emit)
+                    serves = precision == "mixed" or (init == "none" and not checked)
+                    assert bool(op._args.launch_flags & nat.LAUNCH_PDL) == (k >= 8 or serves if pdl is None else pdl)
