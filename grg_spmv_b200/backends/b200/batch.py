@@ -158,11 +158,17 @@ class B200BatchedMatmul:
         mixed = self.precision == "mixed"
         self._release_tiles()
         streams = []
-        for g in self._groups:
+        widths = [(g, self._tile_widths(g.k_total, tile_k)) for g in self._groups]
+        itemsize = rt.layout.dtype.itemsize
+        # padded state rows where they leave the device half of its room, as in the runtime
+        # (not asked under a caller's capture)
+        padded = mixed or (not rt._capturing() and rt._leaves_room(sum(
+            rt._artifacts[g.artifact_index].state.num_nodes * state_ld(w, itemsize) * itemsize for g, ws in widths for w in ws)))
+        for g, ws in widths:
             art = rt._artifacts[g.artifact_index]
             st = art.state
             c0 = 0
-            for w in self._tile_widths(g.k_total, tile_k):
+            for w in ws:
                 if mixed:
                     state = torch.zeros(nat.mix_bytes(st.num_nodes, nat.mix_ld(w)), device=rt.device, dtype=torch.uint8)
                     scratch = None
@@ -170,7 +176,7 @@ class B200BatchedMatmul:
                         nbytes = nat.mix_bytes(st.num_mutations, nat.mix_ld(w)) * (2 if g.use_miss else 1)
                         scratch = torch.zeros(nbytes, device=rt.device, dtype=torch.uint8)
                 else:
-                    state = torch.zeros(st.num_nodes * state_ld(w, rt.layout.dtype.itemsize), device=rt.device, dtype=self._tdt)
+                    state = torch.zeros(st.num_nodes * (state_ld(w, itemsize) if padded else w), device=rt.device, dtype=self._tdt)
                     scratch = None
                 spec = CudaMatmulSpec(direction=g.direction, k=w, emit_all_nodes=False, by_individual=False,
                                       init_mode=InitMode.NONE, backend_init_mode=InitMode.NONE, use_miss=g.use_miss,

@@ -235,7 +235,9 @@ class B200Runtime:
                     if lay.mix_scratch_bytes:
                         self._mix_scratch = torch.zeros(lay.mix_scratch_bytes, device=self.device, dtype=torch.uint8)
                 else:
-                    self._state = torch.zeros(lay.max_num_nodes * lay.state_ld, device=self.device, dtype=tdt)
+                    # without padding where the device would be more than half full: what fitted without still does
+                    ld = lay.state_ld if lay.state_ld == max_k or self._leaves_room(lay.bytes_total) else max_k
+                    self._state = torch.zeros(lay.max_num_nodes * ld, device=self.device, dtype=tdt)
                 self._io0 = torch.zeros((max(lay.max_num_samples, lay.max_num_mutations), max_k), device=self.device, dtype=tdt)
                 io1_rows = side_io_rows(lay.pair, lay.requirements, max_num_mutations=lay.max_num_mutations,
                                         max_num_nodes=lay.max_num_nodes)
@@ -263,6 +265,13 @@ class B200Runtime:
         except Exception:
             self._release()
             raise
+
+    def _leaves_room(self, nbytes: int) -> bool:
+        """Whether ``nbytes`` take at most half of what this process can still allocate on the device."""
+        import torch
+
+        cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        return 2 * int(nbytes) <= torch.cuda.mem_get_info(self.device)[0] + cached
 
     def __exit__(self, exc_type, exc, tb) -> None:
         self._release()
