@@ -458,6 +458,29 @@ class B200Runtime:
     def _torch_caller_stream(self):
         return self._caller_stream
 
+    def _copy_to_host(self, src) -> np.ndarray:
+        """A (k, n) view of a call's result as a NumPy array, on the current stream.  Its rows are
+        put in order on the device, in the node state, which the call is done with: no device
+        memory beside the layout's, and no pass over the result on the host."""
+        import torch
+
+        k, n = src.shape
+        out = np.empty((k, n), dtype=self.layout.dtype)
+        host = torch.from_numpy(out)
+        stage = self._state if self._state.dtype == src.dtype else self._state.view(src.dtype)
+        rows = stage.numel() // n  # of the result at once; a row longer than the state goes in pieces
+        if rows >= k:
+            host.copy_(stage[:k * n].view(k, n).copy_(src))
+            return out
+        cols = n if rows else stage.numel()
+        for r in range(0, k, max(rows, 1)):
+            for c in range(0, n, cols):
+                block = src[r:r + max(rows, 1), c:c + cols]
+                piece = stage[:block.numel()].view(block.shape)
+                piece.copy_(block)
+                host[r:r + max(rows, 1), c:c + cols].copy_(piece)
+        return out
+
     def _begin_call(self) -> None:
         if not self._entered:
             raise RuntimeError("B200Runtime must be entered before matmul")

@@ -249,8 +249,11 @@ class BoundGRG:
         if stream is None:
             return src.detach().cpu().numpy().astype(self._dtype, copy=False).copy()
         with torch.cuda.device(src.device), torch.cuda.stream(stream()):
-            host = src.detach().contiguous().cpu()  # rows put in order on the GPU, not by a host copy
-        return host.numpy().astype(self._dtype, copy=False)
+            to_host = getattr(self._runtime, "_copy_to_host", None)
+            if to_host is not None:
+                return to_host(src.detach())
+            host = src.detach().cpu()
+        return host.numpy().astype(self._dtype, copy=False).copy()
 
     def matmul(self, input, direction, emit_all_nodes: bool = False, by_individual: bool = False, init=None, miss=None):
         if not isinstance(input, np.ndarray):
