@@ -624,13 +624,17 @@ class B200Runtime:
             return _Recording(self._lib, args)
 
     def _launch(self, args: nat.TraverseArgs, recording: _Recording | None = None) -> None:
-        if recording is not None:
+        import torch
+
+        if recording is not None and torch.cuda.current_device() == self.device.index:
             status = recording.launch(args, self.stream_ptr)
         else:
-            import torch
-
+            # PyTorch's guard goes back to a device that has no context without making one there
             with torch.cuda.device(self.device):
-                status = self._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(self.stream_ptr))
+                if recording is not None:
+                    status = recording.launch(args, self.stream_ptr)
+                else:
+                    status = self._lib.grg_b200_traverse(ctypes.byref(args), ctypes.c_void_p(self.stream_ptr))
         if status != nat.OK:
             nat.check(self._lib, status, "grg_b200_traverse")
 

@@ -2885,8 +2885,7 @@ int grg_b200_graph_launch(const grg_b200_graph* g, const grg_b200_traverse_args*
 
 int grg_b200_graph_destroy(grg_b200_graph* g) {
     if (!g) return GRG_B200_OK;
-    const DeviceScope scope(g->device);
-    const cudaError_t err = cudaGraphExecDestroy(g->exec);
+    const cudaError_t err = cudaGraphExecDestroy(g->exec);  // on any current device
     delete g;
     return err == cudaSuccess ? (int)GRG_B200_OK : grg_fail(GRG_B200_ERR_CUDA, "cudaGraphExecDestroy failed: %s", cudaGetErrorString(err));
 }
