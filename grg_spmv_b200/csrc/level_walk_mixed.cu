@@ -124,8 +124,9 @@ struct MixedRows {
 }  // namespace
 
 int launch_walk_mixed(const LevelArgs& la, int init_mode, int64_t num_entries, const int64_t* long_counts, bool pdl, cudaStream_t s) {
-    if (la.ld_state >= (int64_t{1} << 32) || la.k >= (int64_t{1} << 24))
-        return grg_fail(GRG_B200_ERR_UNSUPPORTED, "mixed storage: k = %lld is too large", (long long)la.k);
+    // the walk's columns are 32-bit, and a lane may step one pass (up to 128 columns) past k
+    if (la.ld_state >= (int64_t{1} << 32) || la.k > INT32_MAX - 256)
+        return grg_fail(GRG_B200_ERR_UNSUPPORTED, "mixed storage: k = %lld or ld_state = %lld is too large", (long long)la.k, (long long)la.ld_state);
     return la.up ? launch_rows<MixedRows<true>, MixedRows<true>>(la, init_mode, num_entries, long_counts, pdl, s)
                  : launch_rows<MixedRows<false>, MixedRows<false>>(la, init_mode, num_entries, long_counts, pdl, s);
 }

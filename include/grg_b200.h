@@ -73,7 +73,8 @@ typedef enum grg_b200_status {
  * stored value is within 2^-40 of the exact one relative to it (integers up to 2^40 are
  * exact).  Sums are accumulated in FP64 and rounded back once per node.  A mixed buffer of
  * R rows and ld columns (ld a multiple of 4) is uint32 hi[R * ld] followed by uint16
- * lo[R * ld]; see GRG_B200_MIX_BYTES.  Mixed traversals never use exact order.
+ * lo[R * ld]; see GRG_B200_MIX_BYTES.  Mixed traversals never use exact order.  They take k below
+ * 2^31 - 256 and ld_state below 2^32.
  */
 typedef enum grg_b200_dtype { GRG_B200_F64 = 0, GRG_B200_F32 = 1, GRG_B200_MIXED = 2 } grg_b200_dtype;
 

@@ -103,3 +103,26 @@ def test_mixed_down_with_a_state_wider_than_k(artifact):
             hi = part[: M * ld * 4].view(np.uint32).reshape(M, ld)
             lo = part[nat.mix_plane(M * ld * 4):][: M * ld * 2].view(np.uint16).reshape(M, ld)
             assert not hi[:, k:].any() and not lo[:, k:].any()
+
+
+@pytest.mark.parametrize("k", [(1 << 24) - 4, 1 << 24, (1 << 24) + 129])
+def test_mixed_widths_around_2_to_the_24(k):
+    """The widest calls: a graph of two nodes and as many columns as wanted."""
+    from conftest import artifact_path
+    from grg_spmv_b200.backends.b200 import B200Runtime, plan_b200_layout
+
+    path = artifact_path("sparse_selector")
+    oracle = OracleGRG(path)
+    req = RuntimeRequirements(max_k_up=k, max_k_down=k, need_down_miss_input=False, need_up_miss_output=False,
+                              need_init_vector=False, need_init_matrix=False, need_init_xtx=False)
+    layout = plan_b200_layout(artifacts=[str(path)], dtype=np.float64, requirements=req, vram_budget_bytes=0, ring_buffer_size=0,
+                              device=0, stream=0, precision="mixed", emit_all_nodes=False)
+    with B200Runtime(layout, check_bounds=False) as runtime:
+        (grg,) = runtime.grgs
+        for direction, cols in (("up", grg.num_samples), ("down", grg.num_mutations)):
+            weights = torch.from_numpy(oracle.matmul(np.eye(cols), direction)).to("cuda:0")
+            op = grg.prepare_matmul_cuda(direction=direction, k=k)
+            x = torch.arange(k * cols, device="cuda:0", dtype=torch.float64).remainder_(1021.0).view(k, cols)
+            op.input.copy_(x)
+            op()
+            assert torch.equal(op.output, x @ weights)
