@@ -22,7 +22,8 @@ ops' shared ``io0`` buffer).  Metric: edge·RHS/s = steps · 2·E·k / device ti
   down, the mutation and miss input rows read once.  ``traffic`` is the DRAM traffic (read +
   write) of one up-level-1 launch measured by ncu on the same configuration;
   ``traffic_launches`` lists it with down levels 3, 1 and 0, beside this run's own timing
-  and algorithmic bytes of those launches.
+  and algorithmic bytes of those launches (both null for kernels that were not captured: the
+  default row walk).
 * ``cpu_baseline``: the oracle (SciPy restatement of the reference's ReferenceRuntime) on one
   step of the same graph, RHS columns split over one process per host core (up to k), rank 0,
   N=1 only.
@@ -645,7 +646,7 @@ def run_b200(args) -> None:
                                                             np.max(np.abs(got_down_i - ref_down_i)))),
                          "max_abs_value": float(max(np.max(np.abs(ref_up_i)), np.max(np.abs(ref_down_i))))}
 
-    tuned = {d.value: [v, runtime._heavy_variant.get(d)] for d, v in runtime._variant.items()}
+    tuned = {d.value: "row walk" if runtime._row_walk.get(d) else [v, runtime._heavy_variant.get(d)] for d, v in runtime._variant.items()}
     heavy_used = {"up": int(up._args.heavy_variant), "down": int(down._args.heavy_variant)}
     narrow_used = {"up": int(up._args.narrow_variant), "down": int(down._args.narrow_variant)}
     runtime.__exit__(None, None, None)
@@ -726,7 +727,7 @@ def run_b200(args) -> None:
                        "vram_budget_frac": args.budget_frac, "streamed_bytes_per_step": int(streamed_bytes),
                        "ring_slots": layout.allocated_ring_buffer_size},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": traffic, "traffic_unit": "DRAM bytes of one launch: up level 1 (level_entry_pre_kernel)",
+                         "traffic": traffic, "traffic_unit": "DRAM bytes of one launch: up level 1 (level_entry_pre_kernel)" if traffic is not None else None,
                          "traffic_source": TRAFFIC_SOURCE if traffic is not None else None,
                          "traffic_launches": traffic_launches, "kernel": ("dataflow traversal (sentinel fill + persistent gather kernel + seed/output), per direction"
                                     if pair.plan_down.schedule == "dataflow" else

@@ -1554,7 +1554,7 @@ __device__ __forceinline__ Quad mx_state_row(const OutArgs& a, int64_t n, int64_
 }
 
 // One row per lane group, its extent and first index loaded before the wait.  Four rows, as
-// gather_out_kernel takes, lose here to the decoding's registers (1.5M nodes up k = 31: 525 -> 541 us).
+// gather_out_kernel takes, lose here to the decoding's registers (1.5M nodes, up k = 32: 0.5% of the call).
 template <bool BIAS_PER_ENTRY>
 __global__ void __launch_bounds__(256) gather_out_mx_kernel(OutArgs a) {
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
