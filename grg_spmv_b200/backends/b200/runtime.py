@@ -468,10 +468,10 @@ class B200Runtime:
         out = np.empty((k, n), dtype=self.layout.dtype)
         host = torch.from_numpy(out)
         stage = self._state if self._state.dtype == src.dtype else self._state.view(src.dtype)
-        rows = stage.numel() // n  # of the result at once; a row longer than the state goes in pieces
-        if rows >= k:
+        if k * n <= stage.numel():
             host.copy_(stage[:k * n].view(k, n).copy_(src))
             return out
+        rows = stage.numel() // n  # of the result at once; a row longer than the state goes in pieces
         cols = n if rows else stage.numel()
         for r in range(0, k, max(rows, 1)):
             for c in range(0, n, cols):
